@@ -1,11 +1,12 @@
-// Token mixers of bf16 ragged steps on the tensor pipe (mma.sync; the tiles are too small and too irregular for
-// tcgen05): attention over the paged pools, for prompt portions and for decoded tokens (a long window cut over several
-// CTAs), and retention inside prompt portions, a chunk of positions at a time.
+// Token mixers of bf16 ragged steps on mma.sync: attention over the paged pools, for decoded tokens (a long window cut over
+// several CTAs; sixteen rows are too few for tcgen05) and for prompt portions of sizes attend_portions.cu does not take, and
+// retention inside prompt portions, a chunk of positions at a time.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <cmath>
 
+#include "attend.cuh"
 #include "element.cuh"
 #include "mixers.cuh"
 #include "mma.cuh"
@@ -18,27 +19,6 @@ namespace {
 
 // ---- attention ---------------------------------------------------------------------------------------------------------
 constexpr int kKeys = 64;   // keys per block
-
-struct AttendParams {
-  const bf16* proj;
-  bf16* k_pool;
-  bf16* v_pool;
-  bf16* out;
-  float* part;
-  unsigned* count;
-  const float *q_norm, *k_norm;
-  int proj_stride, out_stride, heads, kv_heads, dim, vdim, pool_dim, v_pool_dim, window, keep, splits, gate_at;
-  int subs, sub_heads;      // query heads of one key head are served in `subs` units of up to `sub_heads`
-  int q_head;               // elements from one query head to the next
-  const int* context;       // portions whose keys and values are rows [.. + position] of k_pool and v_pool (see AttendContext), or null
-  int context_stride;
-  float scale_log2, sink_log2, eps;
-  bool value_is_key, even;
-  Rotary rotary;
-  Blend blend;
-  const float* sinks;
-  __device__ float sink_of(int head) const { return sinks ? sinks[head] * 1.4426950408889634f : sink_log2; }
-};
 
 template <int DT, int WM> struct AttendShape {
   static constexpr int kThreads = WM == 1 ? 128 : 32 * WM;
@@ -758,6 +738,9 @@ template <int DT> int AttendWith(const Queue& q, const StepRows& r, const Attent
     if (status != 0) return status;
   }
   if (r.singles < r.entries) {
+    bool done = false;
+    const int status = AttendPortions(q, r, p, a.k_map, a.v_map, &done);
+    if (status != 0 || done) return status;
     p.splits = 1;
     const int per_tile = 128 / p.sub_heads;
     return LaunchAttend<DT, 8>(q, r, p, (r.longest + per_tile - 1) / per_tile);
@@ -840,6 +823,9 @@ int AttendContext(const Queue& q, const StepRows& r, const AttentionArgs& a, int
   p.context = context;
   p.context_stride = context_stride;
   p.splits = 1;
+  bool done = false;
+  const int status = AttendPortions(q, r, p, a.k_map, a.v_map, &done);
+  if (status != 0 || done) return status;
   const int tiles = (std::max(a.dim, a.vdim) + 15) / 16, per_tile = 128 / p.sub_heads, x = (r.longest + per_tile - 1) / per_tile;
   return tiles <= 2 ? LaunchAttend<2, 8>(q, r, p, x) : tiles <= 4 ? LaunchAttend<4, 8>(q, r, p, x) : tiles <= 6 ? LaunchAttend<6, 8>(q, r, p, x)
          : tiles <= 8 ? LaunchAttend<8, 8>(q, r, p, x) : tiles <= 12 ? LaunchAttend<12, 8>(q, r, p, x) : LaunchAttend<16, 8>(q, r, p, x);
@@ -858,7 +844,7 @@ int PrepareMixers() {
   if (err == cudaSuccess) err = Raise<8>();
   if (err == cudaSuccess) err = Raise<12>();
   if (err == cudaSuccess) err = Raise<16>();
-  return int(err);
+  return err == cudaSuccess ? PreparePortions() : int(err);
 }
 
 }  // namespace tmb

@@ -268,6 +268,7 @@ struct AttentionArgs {
   size_t part_floats;
   unsigned* count;           // arrival counters, zero between launches
   int count_words;
+  const CUtensorMap *k_map, *v_map;   // bf16: EncodePool (or EncodeContext) of keys and values, or null
 };
 // Norms and rotates q in place and appends such k, and v, to the pools. (bf16: rows of portions only; a decoded token's attention
 // does it itself.)
@@ -279,6 +280,10 @@ int AttendTiles(const Queue& q, const StepRows& r, const AttentionArgs& a);   //
 // v_pool + g * v_pool_dim. Query heads are q_head elements apart; nothing is rotated, normed or appended.
 int AttendContext(const Queue& q, const StepRows& r, const AttentionArgs& a, int q_head, const int* context, int context_stride);
 int PrepareMixers();
+// Maps of a pool of `heads` x 16 rows (heads of all blocks) of `dim` columns, and of `count` rows of `heads` x `dim` columns, `stride`
+// elements apart.
+bool EncodePool(CUtensorMap* map, const void* pool, uint64_t heads, uint64_t dim);
+bool EncodeContext(CUtensorMap* map, const void* rows, uint64_t heads, uint64_t dim, uint64_t count, uint64_t stride);
 
 // Attention whose keys and values are images, per head, of one cached latent row per token: scores and sums are taken
 // against the latent rows themselves, with queries `q` already multiplied by their heads' key matrices; `out` rows are the

@@ -63,9 +63,16 @@ struct RaggedPlan {
     LinearMaps in, out, gate_up, down, router;   // (gate_up, down: of the gated unit or of the experts)
     LinearMaps shared_up, shared_down, key_up, value_up, expand, query_up, decay_up, side_gate, side_proj;
     CUtensorMap lookup;
+    CUtensorMap seen_keys, seen_values;      // expanded latent rows
+    bool seen = false;                       // (these can be had)
   };
   std::vector<Maps> maps;      // per layer (bf16 plans)
+  struct PoolMaps {
+    CUtensorMap keys, values;
+    bool there = false;
+  };
   std::vector<CUtensorMap> latent;   // per run (bf16 plans): pools of latent rows
+  std::vector<PoolMaps> pools;       // ... of keys and values
   LinearMaps head;
   // recorded steps of single-row entries, by (entries, wanted, feed)
   std::map<std::tuple<uint32_t, uint32_t, bool>, cudaGraphExec_t> graphs;
@@ -422,6 +429,10 @@ int Enqueue(RaggedPlan* plan, uint32_t entries, uint32_t rows, uint32_t longest,
         seen.gate_at = -1;
         seen.window = m.window;
         seen.scale = a.scale;
+        if (maps->seen) {
+          seen.k_map = &maps->seen_keys;
+          seen.v_map = &maps->seen_values;
+        }
         TMB_TRY(AttendContext(q, r, seen, m.head_stride(), plan->context_at, columns));
       }
     } else {
@@ -456,6 +467,10 @@ int Enqueue(RaggedPlan* plan, uint32_t entries, uint32_t rows, uint32_t longest,
       a.part_floats = plan->part_floats;
       a.count = plan->count;
       a.count_words = plan->count_words;
+      if (maps && plan->pools[i].there) {
+        a.k_map = &plan->pools[i].keys;
+        a.v_map = &plan->pools[i].values;
+      }
       TMB_TRY(RotateAppend(q, r, a));
       TMB_TRY(Attend(q, r, a));
     }
@@ -762,6 +777,24 @@ RaggedPlan* RaggedCreate(const RaggedSpec& spec, const std::vector<void*>& buffe
         ok = ok && EncodeLinear(&maps.gate_up, at(layer.gate_up), uint64_t(mlp.packed_rows()), plan->normed, rows, W8) &&
              EncodeLinear(&maps.down, at(layer.down), uint64_t(spec.width), plan->mlp, rows, uint64_t(padded_columns(mlp.ff)));
       if (!ok) return fail("cuTensorMapEncodeTiled rejected a layer's buffers");
+    }
+    // (the kernels that read portions' keys through maps have a counterpart for what no map can be had of)
+    for (size_t i = 0; i < spec.layers.size(); ++i) {
+      const RaggedMixer& m = spec.layers[i].mixer;
+      RaggedPlan::Maps& maps = plan->maps[i];
+      if (m.kind != RaggedMixer::kLatent || !context_rows) continue;
+      const uint64_t columns = uint64_t(m.expanded_columns()), heads = uint64_t(m.heads);
+      maps.seen = EncodeContext(&maps.seen_keys, plan->expanded, heads, uint64_t(m.expanded_key()), context_rows, columns) &&
+                  EncodeContext(&maps.seen_values, static_cast<char*>(plan->expanded) + heads * m.expanded_key() * 2, heads, uint64_t(m.v_pool_dim()),
+                                context_rows, columns);
+    }
+    plan->pools.resize(spec.runs.size());
+    for (size_t i = 0; i < spec.runs.size(); ++i) {
+      const RaggedMixer& m = spec.layers[size_t(spec.runs[i].layer)].mixer;
+      if (m.kind != RaggedMixer::kAttention) continue;
+      const uint64_t heads = uint64_t(spec.num_blocks) * m.kv_heads;
+      plan->pools[i].there = EncodePool(&plan->pools[i].keys, at(spec.runs[i].k_pool), heads, uint64_t(m.pool_dim())) &&
+                             EncodePool(&plan->pools[i].values, at(spec.runs[i].v_pool), heads, uint64_t(m.v_pool_dim()));
     }
     plan->latent.resize(spec.runs.size());
     for (size_t i = 0; i < spec.runs.size(); ++i) {
