@@ -4,6 +4,7 @@
 
 #include "attend.cuh"
 #include "tensor_map.h"
+#include "umma.cuh"
 
 namespace tmb {
 namespace {
@@ -25,46 +26,6 @@ template <int KC, int VC, int TILES> struct PortionShape {
   static constexpr int kColumns = TILES == 2 ? 512 : 256;
   static constexpr int kSums = 128 * TILES;                                  // first column of the weighted sums
 };
-
-// Products of one step of 16 columns, as umma_bf16, with the descriptors' words apart: the low ones differ between steps by a
-// constant (an issuing thread that builds each descriptor anew is slower than the tensor pipe), the high ones never.
-__device__ __forceinline__ void umma_step(uint32_t d, uint32_t a_low, uint32_t b_low, uint32_t high, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n"
-      " .reg .pred p;\n"
-      " .reg .b64 a, b;\n"
-      " mov.b64 a, {%1, %3};\n"
-      " mov.b64 b, {%2, %3};\n"
-      " setp.ne.b32 p, %5, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n"
-      "}\n" ::"r"(d),
-      "r"(a_low), "r"(b_low), "r"(high), "r"(idesc), "r"(uint32_t(accumulate))
-      : "memory");
-}
-// The same with A in tensor memory: a row a lane, two bf16 a column.
-__device__ __forceinline__ void umma_step_tmem(uint32_t d, uint32_t a, uint32_t b_low, uint32_t high, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n"
-      " .reg .pred p;\n"
-      " .reg .b64 b;\n"
-      " mov.b64 b, {%2, %3};\n"
-      " setp.ne.b32 p, %5, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n"
-      "}\n" ::"r"(d),
-      "r"(a), "r"(b_low), "r"(high), "r"(idesc), "r"(uint32_t(accumulate))
-      : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t elected;
-  asm volatile(
-      "{\n"
-      " .reg .pred p;\n"
-      " elect.sync _|p, 0xffffffff;\n"
-      " selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(elected));
-  return elected != 0;
-}
 
 // Tensor memory by 32 columns, with the wait apart, so that several are in flight; what was loaded may be used behind
 // loads_done() and loaded().

@@ -14,6 +14,7 @@
 #include "ops.h"
 #include "ptx.cuh"
 #include "tensor_map.h"
+#include "umma.cuh"
 
 namespace tmb {
 namespace {
@@ -51,13 +52,12 @@ __host__ __device__ constexpr bool PerExpert(int epilogue) {
 __host__ __device__ constexpr bool IsGlu(int epilogue) { return epilogue == kLinearGlu || epilogue == kLinearExpertGlu; }
 
 template <int BN> struct LinearShape {
-  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 3 : BN == 64 ? 4 : 5;   // about 100 KB (two CTAs per SM), 192 KB for the widest
+  static constexpr int kStages = BN == 128 ? 3 : BN == 64 ? 4 : 5;   // about 100 KB (two CTAs per SM)
   static constexpr int kTokenBytes = BN * kStepK * 2;
   static constexpr int kStageBytes = kWeightBytes + kTokenBytes;
   static constexpr int kSmem = kStages * kStageBytes + 1024 + 256;
   static constexpr int kTmemCols = BN < 32 ? 32 : BN;
-  static constexpr bool kStaged = BN <= 128;   // the epilogue goes through shared memory (needed to sum K splits)
-  static_assert(!kStaged || kStages * kStageBytes >= kRowsM * BN * 4, "the fp32 tile must fit the stages");
+  static_assert(kStages * kStageBytes >= kRowsM * BN * 4, "the fp32 tile must fit the stages");
 };
 
 // gelu(g) = g (1 + tanh(z)) / 2 = g / (1 + exp(-2 z)), z = sqrt(2 / pi) (g + 0.044715 g^3)
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kLinearThreads) linear_tiles(const __grid_cons
     tcgen05_fence_after();
     allow_dependents();
   }
-  if constexpr (Shape::kStaged) {
+  {
     float* tile = reinterpret_cast<float*>(tiles);    // [BN][128]: every stage has been consumed
     if (worker >= 0) {
       constexpr int W = BN >= 64 ? 32 : BN == 32 ? 16 : 8;
@@ -349,70 +349,261 @@ __global__ void __launch_bounds__(kLinearThreads) linear_tiles(const __grid_cons
       }
     }
     if (splits > 1) cluster_sync();   // the peers have read this CTA's tile
-  } else if (worker >= 0 && ok) {
-    const int n = n0 + 32 * quarter + lane;
-    const float bias = g.bias && n < g.n ? g.bias[n] : 0.f;
-    for (int c = column_half * (BN / 2); c < (column_half + 1) * (BN / 2); c += 32) {
-      if (t0 + c >= t_end) break;
-      float v[32];
-      tmem_load_32(tmem + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
-      const int cols = min(32, t_end - t0 - c);
-      if constexpr (IsGlu(EPI)) {
-        const bool upper = lane >= kGluUnit;          // lanes 0..15 hold gate rows, 16..31 the matching up rows
-        const int out = (n0 + 32 * quarter) / 2 + (lane & (kGluUnit - 1));
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {             // lower lanes finish column i, upper lanes column i + 1
-          const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + 1], kGluUnit);
-          const float y = glu_value(upper ? other : v[i], upper ? v[i + 1] : other, g.glu);
-          const int col = i + (upper ? 1 : 0);
-          if (out < g.outputs && col < cols)
-            static_cast<__nv_bfloat16*>(g.out)[size_t(t0 + c + col) * g.out_stride + out] = __float2bfloat16_rn(y);
-        }
-      } else if constexpr (EPI == kLinearRotate) {
-        const Turn turn = turn_of(g.rotate, n);
-        if (__any_sync(0xffffffffu, turn.on)) {
-#pragma unroll
-          for (int i0 = 0; i0 < 32; i0 += 8) {
-            float2 angle[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) angle[i] = angle_at(g.rotate, turn, t0 + c + min(i0 + i, cols - 1));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i0 + i] = turned(turn, angle[i], v[i0 + i], __shfl_xor_sync(0xffffffffu, v[i0 + i], 1));
-          }
-        }
-        if (n < g.n) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (i < cols) emit<EPI>(g, t0 + c + i, n, v[i]);
-        }
-      } else if (n < g.n) {
-        if constexpr (EPI == kLinearAdd) {
-          float* x = static_cast<float*>(g.out) + size_t(t0 + c) * g.out_stride + n;
-          float old[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (i < cols) old[i] = x[size_t(i) * g.out_stride];
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (i < cols) x[size_t(i) * g.out_stride] = old[i] + (v[i] + bias);
-        } else {
-          if (EPI == kLinearStore && n0 < g.tanh_below) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (n < g.tanh_below) v[i] = tanh16(v[i] + bias) - bias;
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (i < cols) emit<EPI>(g, t0 + c + i, out_at + n, v[i] + bias);
-        }
-      }
-    }
   }
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem, Shape::kTmemCols);
+  }
+}
+
+// ---- 256 tokens wide -----------------------------------------------------------------------------------------------------
+// The same product for long prompts: tiles of 128 weight rows x 256 tokens (per expert: as many as it has, up to 256), a CTA an SM,
+// which takes every gridDim.x-th tile. Tensor memory holds two accumulators, so one tile's epilogue runs under the next one's
+// products, and the copies never stop between tiles. Tiles are counted tokens first, per expert weight rows first, as in
+// linear_tiles.
+//
+// PAIR (all but experts): the two CTAs of a cluster work on 256 weight rows x 256 tokens together. Each brings its own 128 weight rows
+// and 128 of the tokens, the first issues the products of both, and each has the sums of its weight rows. A chunk of K then costs a CTA
+// 32 KB instead of 48, which is what L2 can deliver at the tensor pipe's pace. Bound by the tensor pipe and by the last round of tiles
+// (256 tiles over 74 pairs are four rounds for three and a half). 2048 tokens, width 4096: gated unit of 28672 rows 321 us (1.50 PFLOP/s, 0.91
+// of the measured cuBLAS rate) where single tiles of a CTA each took 431; projection of 10240 rows 120 for 150; outputs of K 4096 and 14336
+// 121 for 133 on average. Experts: 128 of 1152 x 2048 with some 128 rows each 164 and 147 us for 169 and 190 (their weights alone are 94 us of
+// copying), because an expert of 129 to 256 rows now reads its weights once.
+constexpr int kWide = 256;
+template <bool PAIR> struct WideShape {
+  static constexpr int kTokens = PAIR ? kWide / 2 : kWide;             // whose rows a CTA brings
+  static constexpr int kStages = PAIR ? 6 : 4, kStageBytes = kWeightBytes + kTokens * kStepK * 2;
+  static constexpr int kSmem = kStages * kStageBytes + 1024;
+};
+
+struct WideTile {
+  int n0, t0, t_end, weight_row, k_at, out_at, columns;
+};
+
+template <int EPI> __device__ __forceinline__ WideTile wide_tile(const LinearParams& g, int i, int token_tiles, int weight_tiles, int t_there) {
+  WideTile tile{};
+  constexpr int kRows = PerExpert(EPI) ? kRowsM : 2 * kRowsM;          // weight rows of a tile
+  if constexpr (PerExpert(EPI)) {
+    const ExpertTile e = g.slots.tiles[i / weight_tiles];
+    tile.n0 = i % weight_tiles * kRowsM;
+    tile.t0 = e.first;
+    tile.t_end = e.first + min(e.count, kWide);
+    tile.weight_row = e.expert * g.n + tile.n0;
+    tile.columns = (tile.t_end - tile.t0 + 15) / 16 * 16;
+  } else {
+    const int w = i / token_tiles;
+    tile.t0 = i % token_tiles * kWide;
+    tile.t_end = t_there;
+    tile.n0 = tile.weight_row = w * kRows + int(cluster_rank()) * kRowsM;
+    tile.columns = kWide;
+    if constexpr (EPI == kLinearHeads) {
+      const int per_head = (g.n + kRows - 1) / kRows, head = w / per_head;
+      tile.n0 = w % per_head * kRows + int(cluster_rank()) * kRowsM;
+      tile.weight_row = head * g.n + tile.n0;
+      tile.k_at = head * g.head_in;
+      tile.out_at = head * g.head_out;
+    }
+  }
+  return tile;
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap tmap,
+                                                                 const LinearParams g, int weight_tiles) {
+  constexpr bool PAIR = !PerExpert(EPI);
+  using Shape = WideShape<PAIR>;
+  constexpr int S = Shape::kStages, kCtas = PAIR ? 2 : 1;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t full[S], empty[S], sum_full[2], sum_empty[2];     // (pairs: full and sum_empty are the first CTA's)
+  __shared__ uint32_t tmem_slot;
+  unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t rank = PAIR ? cluster_rank() : 0;
+  // (tables of tiles and counts of rows were written before the kernel in front of this one, see linear_tiles)
+  int t_there = g.t;
+  if (EPI == kLinearStore && g.rows_there) t_there = min(t_there, *g.rows_there);
+  const int token_tiles = PerExpert(EPI) ? *g.slots.tile_count : (t_there + kWide - 1) / kWide;
+  const int tiles = token_tiles * weight_tiles, first = blockIdx.x / kCtas, step = gridDim.x / kCtas;
+  if (first >= tiles) {
+    dependency_wait();
+    return;
+  }
+  if (threadIdx.x == 0) {
+    prefetch_map(&wmap);
+    prefetch_map(&tmap);
+    for (int s = 0; s < S; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
+    for (int s = 0; s < 2; ++s) mbar_init(&sum_full[s], 1), mbar_init(&sum_empty[s], 256 * kCtas);
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    if constexpr (PAIR) tmem_alloc_pair(&tmem_slot, 512);
+    else tmem_alloc(&tmem_slot, 512);
+  }
+  tcgen05_fence_before();
+  if constexpr (PAIR) cluster_sync();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+
+  if (warp == 0) {
+    if (lane == 0) {
+      constexpr int kBoxes = PerExpert(EPI) ? kWide / 32 : 1;      // (per expert by 32 rows: only those there cost anything)
+      constexpr int kBoxBytes = Shape::kTokens / kBoxes * kStepK * 2;
+      int c = 0, issued = 0;                          // chunks so far
+      bool ok = true, waited = false;
+      auto load = [&](unsigned char* to, const CUtensorMap* map, int x, int y, int s) {
+        if constexpr (PAIR) tma_load_2d_pair(to, map, x, y, &full[s]);
+        else tma_load_2d(to, map, x, y, &full[s]);
+      };
+      auto weights = [&](const WideTile& tile, int chunk, int s, int boxes) {
+        if (rank == 0) mbar_expect_tx(&full[s], uint32_t(kCtas * (kWeightBytes + boxes * kBoxBytes)));
+        load(stages + s * Shape::kStageBytes, &wmap, chunk * kStepK, tile.weight_row, s);
+      };
+      for (int i = first; i < tiles && ok; i += step) {
+        const WideTile tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
+        const int boxes = PerExpert(EPI) ? (tile.t_end - tile.t0 + 31) / 32 : 1, row0 = tile.t0 + int(rank) * Shape::kTokens;
+        int early = 0;
+        if (!waited) {                                // weights do not depend on the kernel before this one
+          for (; early < min(S, g.chunks); ++early) weights(tile, early, early, boxes);
+          dependency_wait();
+          waited = true;
+        }
+        for (int chunk = 0; chunk < g.chunks; ++chunk, ++c) {
+          const int s = c % S;
+          if (c >= S) ok = wait_bounded(&empty[s], uint32_t((c / S) - 1) & 1u, g.status, 1);
+          if (!ok) break;
+          if (c >= early) weights(tile, chunk, s, boxes);
+          unsigned char* rows = stages + s * Shape::kStageBytes + kWeightBytes;
+          for (int j = 0; j < boxes; ++j) load(rows + j * kBoxBytes, &tmap, tile.k_at + chunk * kStepK, row0 + j * (Shape::kTokens / kBoxes), s);
+          issued = c + 1;
+        }
+      }
+      if (!ok && rank == 0)   // leaving early: let the copies already issued land first
+        for (int j = issued > S ? issued - S : 0; j < issued; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
+    }
+  } else if (warp == 1) {
+    // the warp walks along together, one lane issues
+    const uint64_t desc = umma_desc_k_sw128(smem_u32(stages), 1024);
+    const uint32_t low = uint32_t(desc), high = uint32_t(desc >> 32);
+    int c = 0, k = 0;
+    bool ok = true;
+    for (int i = first; i < tiles && ok && rank == 0; i += step, ++k) {
+      const int columns = PerExpert(EPI) ? __shfl_sync(0xffffffffu, wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there).columns, 0) : kWide;
+      const uint32_t idesc = umma_idesc_bf16(kCtas * kRowsM, columns), sum = tmem + (k & 1) * kWide;
+      if (k > 1) ok = __all_sync(0xffffffffu, wait_bounded(&sum_empty[k & 1], uint32_t((k >> 1) - 1) & 1u, g.status, 3));
+      if (!ok) break;
+      tcgen05_fence_after();
+      for (int chunk = 0; chunk < g.chunks; ++chunk, ++c) {
+        const int s = c % S;
+        ok = __all_sync(0xffffffffu, wait_bounded(&full[s], uint32_t(c / S) & 1u, g.status, 3));
+        if (!ok) break;
+        tcgen05_fence_after();
+        if (elect_one()) {
+          const uint32_t w = low + s * (Shape::kStageBytes / 16), t = w + kWeightBytes / 16;
+#pragma unroll
+          for (int j = 0; j < kStepK / 16; ++j) {
+            if constexpr (PAIR) umma_step_pair(sum, w + 2 * j, t + 2 * j, high, idesc, (chunk | j) != 0);
+            else umma_step(sum, w + 2 * j, t + 2 * j, high, idesc, (chunk | j) != 0);
+          }
+          if constexpr (PAIR) umma_commit_pair(&empty[s]);
+          else umma_commit(&empty[s]);
+        }
+        __syncwarp();
+      }
+      if (elect_one()) {                              // arrives once everything issued above is done
+        if constexpr (PAIR) umma_commit_pair(&sum_full[k & 1]);
+        else umma_commit(&sum_full[k & 1]);
+      }
+      __syncwarp();
+    }
+    if (!ok)
+      for (int j = 0; j < 1000000 && !mbar_try_wait(&sum_full[k & 1], uint32_t(k >> 1) & 1u); ++j) {
+      }
+  } else {
+    const int quarter = warp & 3, column_half = (warp - 2) >> 2;
+    bool ok = true, waited = false;
+    int k = 0;
+    for (int i = first; i < tiles; i += step, ++k) {
+      const WideTile tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
+      const int n0 = tile.n0, t0 = tile.t0, t_end = tile.t_end, out_at = tile.out_at;
+      if (!waited) dependency_wait();
+      waited = true;
+      ok = __all_sync(0xffffffffu, wait_bounded(&sum_full[k & 1], uint32_t(k >> 1) & 1u, g.status, 4));
+      if (!ok) break;
+      tcgen05_fence_after();
+      if (i + step >= tiles) allow_dependents();
+      const uint32_t sum = tmem + (k & 1) * kWide;
+      const int n = n0 + 32 * quarter + lane;
+      const float bias = g.bias && n < g.n ? g.bias[n] : 0.f;
+      for (int c = column_half * (kWide / 2); c < (column_half + 1) * (kWide / 2); c += 32) {
+        if (t0 + c >= t_end) break;
+        float v[32];
+        tmem_load_32(sum + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
+        const int cols = min(32, t_end - t0 - c);
+        if constexpr (IsGlu(EPI)) {
+          const bool upper = lane >= kGluUnit;          // lanes 0..15 hold gate rows, 16..31 the matching up rows
+          const int out = (n0 + 32 * quarter) / 2 + (lane & (kGluUnit - 1));
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {             // lower lanes finish column i, upper lanes column i + 1
+            const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + 1], kGluUnit);
+            const float y = glu_value(upper ? other : v[i], upper ? v[i + 1] : other, g.glu);
+            const int col = i + (upper ? 1 : 0);
+            if (out < g.outputs && col < cols)
+              static_cast<__nv_bfloat16*>(g.out)[size_t(t0 + c + col) * g.out_stride + out] = __float2bfloat16_rn(y);
+          }
+        } else if constexpr (EPI == kLinearRotate) {
+          const Turn turn = turn_of(g.rotate, n);
+          if (__any_sync(0xffffffffu, turn.on)) {
+#pragma unroll
+            for (int i0 = 0; i0 < 32; i0 += 8) {
+              float2 angle[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) angle[i] = angle_at(g.rotate, turn, t0 + c + min(i0 + i, cols - 1));
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i0 + i] = turned(turn, angle[i], v[i0 + i], __shfl_xor_sync(0xffffffffu, v[i0 + i], 1));
+            }
+          }
+          if (n < g.n) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < cols) emit<EPI>(g, t0 + c + i, n, v[i]);
+          }
+        } else if (n < g.n) {
+          if constexpr (EPI == kLinearAdd) {
+            float* x = static_cast<float*>(g.out) + size_t(t0 + c) * g.out_stride + n;
+            float old[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < cols) old[i] = x[size_t(i) * g.out_stride];
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < cols) x[size_t(i) * g.out_stride] = old[i] + (v[i] + bias);
+          } else {
+            if (EPI == kLinearStore && n0 < g.tanh_below) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (n < g.tanh_below) v[i] = tanh16(v[i] + bias) - bias;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < cols) emit<EPI>(g, t0 + c + i, out_at + n, v[i] + bias);
+          }
+        }
+      }
+      tcgen05_fence_before();
+      if constexpr (PAIR) arrive_at(&sum_empty[k & 1], 0);
+      else mbar_arrive(&sum_empty[k & 1]);
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if constexpr (PAIR) cluster_sync();                  // (neither is gone while the other still signals it)
+  if (warp == 1) {
+    tcgen05_fence_after();
+    if constexpr (PAIR) tmem_dealloc_pair(tmem, 512);
+    else tmem_dealloc(tmem, 512);
   }
 }
 
@@ -505,6 +696,37 @@ template <int BN> cudaError_t RaiseLimit() {
 // Most tiles the slots of a step can fall into: full ones, and one more for every expert in use.
 int MostTiles(const ExpertSlots& s) { return s.slots / s.tile_rows + std::min(s.experts, s.slots); }
 
+cudaError_t LaunchWide(const Queue& q, const LinearArgs& a, const LinearParams& p) {
+  auto kernel = a.epilogue == kLinearAdd ? linear_wide<kLinearAdd> : a.epilogue == kLinearGlu ? linear_wide<kLinearGlu>
+                : a.epilogue == kLinearFloat ? linear_wide<kLinearFloat> : a.epilogue == kLinearExpertUp ? linear_wide<kLinearExpertUp>
+                : a.epilogue == kLinearExpertDown ? linear_wide<kLinearExpertDown> : a.epilogue == kLinearHeads ? linear_wide<kLinearHeads>
+                : a.epilogue == kLinearExpertGlu ? linear_wide<kLinearExpertGlu> : a.epilogue == kLinearRotate ? linear_wide<kLinearRotate>
+                : a.epilogue == kLinearSide ? linear_wide<kLinearSide> : linear_wide<kLinearStore>;
+  const bool pair = !PerExpert(a.epilogue);
+  const int rows = pair ? 2 * kRowsM : kRowsM, weight_tiles = (a.n + rows - 1) / rows * std::max(a.heads, 1);
+  const long long tiles = (long long)(weight_tiles) * (pair ? (a.t + kWide - 1) / kWide : MostTiles(a.slots));
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(pair ? 2 * unsigned(std::min<long long>(tiles, q.sm_count / 2)) : unsigned(std::min<long long>(tiles, q.sm_count)));
+  config.blockDim = dim3(kLinearThreads);
+  config.dynamicSmemBytes = pair ? WideShape<true>::kSmem : WideShape<false>::kSmem;
+  config.stream = q.stream;
+  cudaLaunchAttribute attributes[2];
+  int count = 0;
+  if (q.chained) {
+    attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[count++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (pair) {
+    attributes[count].id = cudaLaunchAttributeClusterDimension;
+    attributes[count].val.clusterDim.x = 2;
+    attributes[count].val.clusterDim.y = 1;
+    attributes[count++].val.clusterDim.z = 1;
+  }
+  config.attrs = attributes;
+  config.numAttrs = unsigned(count);
+  return cudaLaunchKernelEx(&config, kernel, a.maps->weight, a.maps->rows[pair ? 3 : 1], p, weight_tiles);
+}
+
 template <int BN>
 cudaError_t LaunchTiles(const Queue& q, const LinearArgs& a, const LinearParams& p, int map, int splits) {
   auto kernel = a.epilogue == kLinearAdd ? linear_tiles<BN, kLinearAdd> : a.epilogue == kLinearGlu ? linear_tiles<BN, kLinearGlu>
@@ -568,7 +790,7 @@ int ExpertTileRows(const Queue& q, int slots, int experts) {
   if (q.f32) return kTile32;
   const int share = (slots + experts - 1) / experts;   // slots of an expert on average; most have no more than 4/3 of it
   int rows = 16;
-  while (rows < 128 && rows * 3 < share * 4) rows *= 2;
+  while (rows < kWide && rows * 3 < share * 4) rows *= 2;
   return rows;
 }
 
@@ -577,7 +799,11 @@ int PrepareLinear() {
   if (err == cudaSuccess) err = RaiseLimit<32>();
   if (err == cudaSuccess) err = RaiseLimit<64>();
   if (err == cudaSuccess) err = RaiseLimit<128>();
-  if (err == cudaSuccess) err = RaiseLimit<256>();
+  for (auto kernel : {linear_wide<kLinearStore>, linear_wide<kLinearAdd>, linear_wide<kLinearGlu>, linear_wide<kLinearFloat>, linear_wide<kLinearHeads>,
+                      linear_wide<kLinearRotate>, linear_wide<kLinearSide>})
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<true>::kSmem);
+  for (auto kernel : {linear_wide<kLinearExpertUp>, linear_wide<kLinearExpertDown>, linear_wide<kLinearExpertGlu>})
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<false>::kSmem);
   return int(err);
 }
 
@@ -642,7 +868,7 @@ int Linear(const Queue& q, const LinearArgs& a) {
     case 1: return int(LaunchTiles<32>(q, a, p, 1, splits));
     case 2: return int(LaunchTiles<64>(q, a, p, 2, splits));
     case 3: return int(LaunchTiles<128>(q, a, p, 3, splits));
-    default: return int(LaunchTiles<256>(q, a, p, 4, splits));
+    default: return int(LaunchWide(q, a, p));
   }
 }
 
