@@ -24,6 +24,7 @@
 #include "encoder.h"
 #include "ptx.cuh"
 #include "tensor_map.h"
+#include "umma.cuh"
 
 namespace tmb {
 namespace {
@@ -105,6 +106,36 @@ template <int BN, bool DEEP = false> struct GemmShape {
   static constexpr int kSmem = kStages * kStageBytes + 1024 /* alignment */ + 256 /* barriers */ + 512 /* the tile's bias */;
   static constexpr int kTmemCols = BN < 32 ? 32 : BN;
 };
+
+// W columns of a token's row: fp32 partial sums as they are, or with their bias (column `c` of the tile's on) and the exact
+// (erf) GELU of the BERT feed-forward as 16-bit elements.
+template <typename T, int EPI, int W>
+__device__ __forceinline__ void write_columns(const float (&v)[W], T* out, float* part, size_t at, const unsigned char* bias_tile, int c) {
+  if (EPI == kEpiPartial) {
+#pragma unroll
+    for (int i = 0; i < W / 8; ++i)
+      store_32_bytes(part + at + 8 * i,
+                     make_uint4(__float_as_uint(v[8 * i]), __float_as_uint(v[8 * i + 1]), __float_as_uint(v[8 * i + 2]), __float_as_uint(v[8 * i + 3])),
+                     make_uint4(__float_as_uint(v[8 * i + 4]), __float_as_uint(v[8 * i + 5]), __float_as_uint(v[8 * i + 6]), __float_as_uint(v[8 * i + 7])));
+  } else {
+#pragma unroll
+    for (int i = 0; i < W / 16; ++i) {
+      float lo[8], hi[8];
+      unpack8<T>(reinterpret_cast<const uint4*>(bias_tile)[(c + 16 * i) / 8], lo);
+      unpack8<T>(reinterpret_cast<const uint4*>(bias_tile)[(c + 16 * i) / 8 + 1], hi);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        lo[j] += v[16 * i + j];
+        hi[j] += v[16 * i + 8 + j];
+        if (EPI == kEpiBiasGelu) {
+          lo[j] = 0.5f * lo[j] * (1.0f + erf_fast(lo[j] * 0.70710678118654752f));
+          hi[j] = 0.5f * hi[j] * (1.0f + erf_fast(hi[j] * 0.70710678118654752f));
+        }
+      }
+      store_32_bytes(out + at + 16 * i, pack8<T>(lo), pack8<T>(hi));
+    }
+  }
+}
 
 // C[128 x BN tile] = A[rows x K] (tokens, K-major) * W[N x K]^T (nn.Linear layout, K-major), fp32 in tensor memory.
 // blockIdx = (n tile, m tile, K split). Warp 0: TMA producer. Warp 1: tensor-memory owner and MMA issuer.
@@ -213,32 +244,8 @@ __global__ void __launch_bounds__(kGemmThreads) encoder_gemm(const __grid_consta
         } else {
           tmem_load_16(tmem + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
         }
-        if (EPI == kEpiPartial) {
-          float* dst = static_cast<float*>(g.out) + size_t(blockIdx.z) * g.part_stride + size_t(row) * g.ldc + n0 + c;
-#pragma unroll
-          for (int i = 0; i < W / 8; ++i)
-            store_32_bytes(dst + 8 * i,
-                           make_uint4(__float_as_uint(v[8 * i]), __float_as_uint(v[8 * i + 1]), __float_as_uint(v[8 * i + 2]), __float_as_uint(v[8 * i + 3])),
-                           make_uint4(__float_as_uint(v[8 * i + 4]), __float_as_uint(v[8 * i + 5]), __float_as_uint(v[8 * i + 6]), __float_as_uint(v[8 * i + 7])));
-        } else {
-          T* dst = static_cast<T*>(g.out) + size_t(row) * g.ldc + n0 + c;
-#pragma unroll
-          for (int i = 0; i < W / 16; ++i) {
-            float lo[8], hi[8];
-            unpack8<T>(reinterpret_cast<const uint4*>(bias_tile)[(c + 16 * i) / 8], lo);
-            unpack8<T>(reinterpret_cast<const uint4*>(bias_tile)[(c + 16 * i) / 8 + 1], hi);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              lo[j] += v[16 * i + j];
-              hi[j] += v[16 * i + 8 + j];
-              if (EPI == kEpiBiasGelu) {   // the exact (erf) GELU of the BERT feed-forward
-                lo[j] = 0.5f * lo[j] * (1.0f + erf_fast(lo[j] * 0.70710678118654752f));
-                hi[j] = 0.5f * hi[j] * (1.0f + erf_fast(hi[j] * 0.70710678118654752f));
-              }
-            }
-            store_32_bytes(dst + 16 * i, pack8<T>(lo), pack8<T>(hi));
-          }
-        }
+        write_columns<T, EPI, W>(v, static_cast<T*>(g.out), static_cast<float*>(g.out) + size_t(blockIdx.z) * g.part_stride, size_t(row) * g.ldc + n0 + c,
+                                 bias_tile, c);
       }
     }
   }
@@ -247,6 +254,137 @@ __global__ void __launch_bounds__(kGemmThreads) encoder_gemm(const __grid_consta
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem, Shape::kTmemCols);
+  }
+}
+
+// ---- the same for many rows ----------------------------------------------------------------------------------
+// Tiles of 128 tokens x BN weight rows, a CTA an SM, which takes every gridDim.x-th tile. Tensor memory holds two
+// accumulators, so one tile's epilogue runs under the next one's products, and the copies never stop between tiles.
+// 4096 tokens (32 sequences), hidden 768, against encoder_gemm's tiles of 128 x 128 in a CTA each: FFN up 27 us for 40, QKV 22 for 26, output and FFN
+// down 19 for 21 on average (128 tiles of 192 are one round of CTAs that leaves 20 SMs idle). With 12 chunks of K a tile and two tiles a CTA, its start and
+// its last epilogue are still half of the time.
+template <int BN> struct WideShape {
+  static constexpr int kBBytes = BN * kTileK * 2, kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = BN == 256 ? 4 : BN == 192 ? 5 : 6;
+  static constexpr int kSmem = kStages * kStageBytes + 1024;
+  static constexpr int kAccumulator = BN == 192 ? 256 : BN;   // columns from one accumulator to the other
+};
+
+template <typename T, int BN, int EPI>
+__global__ void __launch_bounds__(kGemmThreads, 1) encoder_wide(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap0,
+                                                       const __grid_constant__ CUtensorMap wmap1, const __grid_constant__ CUtensorMap wmap2,
+                                                       const GemmArgs g, int token_tiles, int tiles) {
+  using Shape = WideShape<BN>;
+  constexpr int S = Shape::kStages, A = Shape::kAccumulator;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t full[S], empty[S], sum_full[2], sum_empty[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ __align__(16) unsigned char bias_tile[2][BN * 2];
+  unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  auto map_of = [&](int n0) { return n0 / g.n_per_map == 0 ? &wmap0 : n0 / g.n_per_map == 1 ? &wmap1 : &wmap2; };
+  if (threadIdx.x == 0) {
+    prefetch_map(&amap);
+    prefetch_map(map_of(int(blockIdx.x) / token_tiles * BN));
+    for (int s = 0; s < S; ++s) mbar_init(&full[s], 1), mbar_init(&empty[s], 1);
+    for (int s = 0; s < 2; ++s) mbar_init(&sum_full[s], 1), mbar_init(&sum_empty[s], 256);
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&tmem_slot, 2 * A);
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int c = 0, issued = 0;
+      bool ok = true, waited = false;
+      for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+        const int n0 = i / token_tiles * BN, m0 = i % token_tiles * kTileM;
+        const CUtensorMap* wmap = map_of(n0);
+        auto weights = [&](int chunk, int s) {
+          mbar_expect_tx(&full[s], Shape::kStageBytes);
+          tma_load_2d(stages + s * Shape::kStageBytes + kABytes, wmap, chunk * kTileK, n0 % g.n_per_map, &full[s]);
+        };
+        int early = 0;
+        if (!waited) {                       // weights do not depend on the kernel before this one
+          for (; early < S && early < g.kchunks; ++early) weights(early, early);
+          dependency_wait();
+          waited = true;
+        }
+        for (int chunk = 0; chunk < g.kchunks; ++chunk, ++c) {
+          const int s = c % S;
+          if (c >= S) ok = wait_bounded(&empty[s], uint32_t((c / S) - 1) & 1u, g.status, 1);
+          if (!ok) break;
+          if (c >= early) weights(chunk, s);
+          tma_load_2d(stages + s * Shape::kStageBytes, &amap, chunk * kTileK, m0, &full[s]);
+          issued = c + 1;
+        }
+      }
+      if (!ok)   // leaving early: first let the copies already issued land in this CTA's shared memory
+        for (int j = issued > S ? issued - S : 0; j < issued; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
+    }
+  } else if (warp == 1) {
+    // the warp walks along together, one lane issues
+    const uint32_t idesc = (1u << 4) | Num<T>::kIdescFormat | (uint32_t(BN >> 3) << 17) | (uint32_t(kTileM >> 4) << 24);
+    const uint64_t desc = umma_desc_k_sw128(smem_u32(stages), 1024);
+    const uint32_t low = uint32_t(desc), high = uint32_t(desc >> 32);
+    int c = 0, k = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x, ++k) {
+      if (k > 1) ok = __all_sync(0xffffffffu, wait_bounded(&sum_empty[k & 1], uint32_t((k >> 1) - 1) & 1u, g.status, 3));
+      if (!ok) break;
+      for (int chunk = 0; chunk < g.kchunks; ++chunk, ++c) {
+        const int s = c % S;
+        ok = __all_sync(0xffffffffu, wait_bounded(&full[s], uint32_t(c / S) & 1u, g.status, 3));
+        if (!ok) break;
+        tcgen05_fence_after();
+        if (elect_one()) {
+          const uint32_t a = low + s * (Shape::kStageBytes / 16), b = a + kABytes / 16;
+#pragma unroll
+          for (int j = 0; j < kTileK / 16; ++j) umma_step(tmem + (k & 1) * A, a + 2 * j, b + 2 * j, high, idesc, (chunk | j) != 0);
+          umma_commit(&empty[s]);
+        }
+        __syncwarp();
+      }
+      if (elect_one()) umma_commit(&sum_full[k & 1]);
+      __syncwarp();
+    }
+    if (!ok)
+      for (int j = 0; j < 1000000 && !mbar_try_wait(&sum_full[k & 1], uint32_t(k >> 1) & 1u); ++j) {
+      }
+  } else {
+    const int quarter = warp & 3, column_half = (warp - 2) >> 2;
+    int k = 0;
+    for (int i = blockIdx.x; i < tiles; i += gridDim.x, ++k) {
+      const int n0 = i / token_tiles * BN, row = i % token_tiles * kTileM + 32 * quarter + lane;
+      if (EPI != kEpiPartial) {              // the tile's bias (weights: no need to wait for the kernel before)
+        const int e = threadIdx.x - 64;
+        if (e < BN / 8)
+          reinterpret_cast<uint4*>(bias_tile[k & 1])[e] =
+              __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(g.bias[n0 / g.n_per_map]) + n0 % g.n_per_map) + e);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+      }
+      if (k == 0) dependency_wait();
+      if (!__all_sync(0xffffffffu, wait_bounded(&sum_full[k & 1], uint32_t(k >> 1) & 1u, g.status, 4))) break;
+      tcgen05_fence_after();
+      if (i + int(gridDim.x) >= tiles) allow_dependents();
+#pragma unroll 1
+      for (int c = column_half * (BN / 2); c < (column_half + 1) * (BN / 2); c += 32) {
+        float v[32];
+        tmem_load_32(tmem + (k & 1) * A + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
+        write_columns<T, EPI, 32>(v, static_cast<T*>(g.out), reinterpret_cast<float*>(g.out), size_t(row) * g.ldc + n0 + c, bias_tile[k & 1], c);
+      }
+      tcgen05_fence_before();
+      mbar_arrive(&sum_empty[k & 1]);
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem, 2 * A);
   }
 }
 
@@ -521,6 +659,7 @@ struct GemmLaunch {
   dim3 grid;
   int bn, epilogue;
   bool dependent, deep;
+  int wide_tiles = 0;      // > 0: so many tiles of encoder_wide
 };
 
 struct EncoderPlan {
@@ -552,7 +691,23 @@ template <typename T, int BN, bool DEEP = false> cudaError_t LaunchGemmTile(cons
   }
 }
 
+template <typename T, int BN, int EPI> cudaError_t LaunchWideAs(const GemmLaunch& l, cudaStream_t stream) {
+  auto kernel = encoder_wide<T, BN, EPI>;
+  if (!stream) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<BN>::kSmem);
+  return Launch(kernel, l.grid, dim3(kGemmThreads), WideShape<BN>::kSmem, stream, l.dependent, l.amap, l.wmap[0], l.wmap[1], l.wmap[2], l.args,
+                l.wide_tiles / (l.args.ldc / BN), l.wide_tiles);
+}
+
+template <typename T, int BN> cudaError_t LaunchWide(const GemmLaunch& l, cudaStream_t stream) {
+  switch (l.epilogue) {
+    case kEpiBias: return LaunchWideAs<T, BN, kEpiBias>(l, stream);
+    case kEpiBiasGelu: return LaunchWideAs<T, BN, kEpiBiasGelu>(l, stream);
+    default: return LaunchWideAs<T, BN, kEpiPartial>(l, stream);
+  }
+}
+
 template <typename T> cudaError_t LaunchGemm(const GemmLaunch& l, cudaStream_t stream) {
+  if (l.wide_tiles) return l.bn == 256 ? LaunchWide<T, 256>(l, stream) : l.bn == 192 ? LaunchWide<T, 192>(l, stream) : LaunchWide<T, 128>(l, stream);
   switch (l.bn) {
     case 128: return LaunchGemmTile<T, 128>(l, stream);
     case 64: return LaunchGemmTile<T, 64>(l, stream);
@@ -593,12 +748,27 @@ void ChooseTiling(int rows, int n, int k, int sm_count, bool may_split, int* bn,
   }
 }
 
+// Width of the tiles of a projection for many rows (encoder_wide), 0: too few of them. A tile's products take as long as its
+// width, and the last round of tiles leaves SMs idle: the width whose rounds end first.
+int WideTiling(int rows, int n, int n_per_map, int sm_count) {
+  const int mtiles = rows / kTileM;
+  if (mtiles * (n / 128) < sm_count) return 0;
+  int best = 0, least = 0;
+  for (int bn : {256, 192, 128}) {
+    if (n_per_map % bn) continue;
+    const int cost = (mtiles * (n / bn) + sm_count - 1) / sm_count * (bn + 16);
+    if (!best || cost < least) best = bn, least = cost;
+  }
+  return best;
+}
+
 // Every instantiation a plan of this element type may launch gets its dynamic shared-memory limit raised.
 template <typename T> cudaError_t PrepareGemms() {
   GemmLaunch l{};
-  for (int form = 0; form < 4; ++form)
+  for (int form = 0; form < 7; ++form)
     for (int epilogue : {int(kEpiBias), int(kEpiBiasGelu), int(kEpiPartial)}) {
-      l.bn = form == 0 ? 128 : form == 1 ? 64 : 32;
+      l.wide_tiles = form >= 4 ? 1 : 0;
+      l.bn = form == 0 || form == 4 ? 128 : form == 1 ? 64 : form == 5 ? 192 : form == 6 ? 256 : 32;
       l.deep = form == 3;
       l.epilogue = epilogue;
       const cudaError_t err = LaunchGemm<T>(l, nullptr);   // a null stream means: prepare only
@@ -663,6 +833,10 @@ template <typename T> cudaError_t Enqueue(EncoderPlan& plan, const PlanSpec& spe
     GemmLaunch l{};
     int splits = 1;
     ChooseTiling(rows, n, k, sm_count, epilogue == kEpiPartial, &l.bn, &splits);
+    if (const int wide = splits == 1 ? WideTiling(rows, n, n_per_map, sm_count) : 0) {
+      l.bn = wide;
+      l.wide_tiles = rows / kTileM * (n / wide);
+    }
     if (!EncodeMatrix(&l.amap, plan.f16, a, uint64_t(rows), uint64_t(k), kTileM)) {
       *error = "cuTensorMapEncodeTiled rejected an activation buffer";
       return cudaErrorInvalidValue;
@@ -679,7 +853,7 @@ template <typename T> cudaError_t Enqueue(EncoderPlan& plan, const PlanSpec& spe
     l.args.kchunks = k / kTileK / splits;
     l.args.part_stride = (unsigned long long)(rows) * n;
     l.args.status = plan.status;
-    l.grid = dim3(unsigned(n / l.bn), unsigned(rows / kTileM), unsigned(splits));
+    l.grid = l.wide_tiles ? dim3(unsigned(std::min(l.wide_tiles, sm_count))) : dim3(unsigned(n / l.bn), unsigned(rows / kTileM), unsigned(splits));
     l.epilogue = epilogue;
     l.deep = l.bn == 32 && int(l.grid.x * l.grid.y * l.grid.z) <= sm_count;
     l.dependent = chained;
