@@ -41,7 +41,7 @@ __device__ __forceinline__ unsigned ordered(float v) {
 // 32 * kMine experts, a lane keeps its own in registers and strikes out what was taken; otherwise every turn takes the
 // largest of those behind the one before it in that order.
 constexpr int kMine = 8;
-template <bool HELD> __device__ __forceinline__ void choose(const RouteArgs& a, int row, int lane) {
+template <bool HELD, bool RANKED> __device__ __forceinline__ void choose(const RouteArgs& a, int row, int lane) {
   const float* z = a.logits + size_t(row) * (a.experts + a.extra);
   unsigned key[kMine];
   if (HELD)
@@ -89,11 +89,12 @@ template <bool HELD> __device__ __forceinline__ void choose(const RouteArgs& a, 
   if (lane < a.top) {
     a.choice[row * a.top + lane] = taken;
     a.score[row * a.top + lane] = score;
+    if (RANKED && a.rank) a.rank[row * a.top + lane] = atomicAdd(&a.tally[taken], 1);
   }
 }
 // The same where scores are not the logits' order: ranked by score + correction, from the best groups only. `line` holds the
 // row's logits, then its ranks (shared memory where HELD, else a.ranks). One warp runs this once, so its loops stay short code.
-template <bool HELD> __device__ __forceinline__ void choose_ranked(const RouteArgs& a, int row, int lane, float* line, const float* correction) {
+template <bool HELD, bool RANKED> __device__ __forceinline__ void choose_ranked(const RouteArgs& a, int row, int lane, float* line, const float* correction) {
   const float* z = a.logits + size_t(row) * (a.experts + a.extra);
   float high = -INFINITY, sum = 0.f;
 #pragma unroll 4
@@ -190,17 +191,43 @@ template <bool HELD> __device__ __forceinline__ void choose_ranked(const RouteAr
   if (lane < a.top) {
     a.choice[row * a.top + lane] = taken;
     a.score[row * a.top + lane] = a.weights ? score / (total + 1e-20f) : score;
+    if (RANKED && a.rank) a.rank[row * a.top + lane] = atomicAdd(&a.tally[taken], 1);
   }
 }
-__device__ __forceinline__ void choose(const RouteArgs& a, int row, int lane, float* line, const float* correction) {
+// RANKED: assignments may be given their places among their expert's (RouteArgs::rank).
+template <bool RANKED> __device__ __forceinline__ void choose(const RouteArgs& a, int row, int lane, float* line, const float* correction) {
   const bool held = a.experts <= 32 * kMine;
   if (a.ranks) {
-    if (held) choose_ranked<true>(a, row, lane, line, correction);
-    else choose_ranked<false>(a, row, lane, a.ranks + size_t(row) * a.experts, correction);
+    if (held) choose_ranked<true, RANKED>(a, row, lane, line, correction);
+    else choose_ranked<false, RANKED>(a, row, lane, a.ranks + size_t(row) * a.experts, correction);
   } else {
-    if (held) choose<true>(a, row, lane);
-    else choose<false>(a, row, lane);
+    if (held) choose<true, RANKED>(a, row, lane);
+    else choose<false, RANKED>(a, row, lane);
   }
+}
+
+// By one warp: every expert's first slot, and the tiles of its slots.
+__device__ __forceinline__ void lay_out_experts(const RouteArgs& a, const int* counts, int* first, int lane) {
+  int slots = 0, tiles = 0;
+  for (int base = 0; base < a.experts; base += 32) {
+    const int e = base + lane, count = e < a.experts ? counts[e] : 0, mine = (count + a.tile_rows - 1) / a.tile_rows;
+    int slot_sum = count, tile_sum = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int s = __shfl_up_sync(0xffffffffu, slot_sum, o), t = __shfl_up_sync(0xffffffffu, tile_sum, o);
+      if (lane >= o) {
+        slot_sum += s;
+        tile_sum += t;
+      }
+    }
+    const int at = slots + slot_sum - count;
+    if (e < a.experts) first[e] = at;
+    for (int t = 0; t < mine; ++t)
+      a.tiles[tiles + tile_sum - mine + t] = {e, at + t * a.tile_rows, min(count - t * a.tile_rows, a.tile_rows), 0};
+    slots += __shfl_sync(0xffffffffu, slot_sum, 31);
+    tiles += __shfl_sync(0xffffffffu, tile_sum, 31);
+  }
+  if (lane == 0) *a.tile_count = tiles;
 }
 
 // The step's assignments sorted by expert, by one CTA. `first` holds every expert's first slot, then its next free one.
@@ -222,28 +249,7 @@ __device__ __forceinline__ void sort_assignments(const RouteArgs& a, int* counts
       if (choice[u] >= 0) atomicAdd(&counts[choice[u]], 1);
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    int slots = 0, tiles = 0;
-    for (int base = 0; base < a.experts; base += 32) {
-      const int e = base + lane, count = e < a.experts ? counts[e] : 0, mine = (count + a.tile_rows - 1) / a.tile_rows;
-      int slot_sum = count, tile_sum = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int s = __shfl_up_sync(0xffffffffu, slot_sum, o), t = __shfl_up_sync(0xffffffffu, tile_sum, o);
-        if (lane >= o) {
-          slot_sum += s;
-          tile_sum += t;
-        }
-      }
-      const int at = slots + slot_sum - count;
-      if (e < a.experts) first[e] = at;
-      for (int t = 0; t < mine; ++t)
-        a.tiles[tiles + tile_sum - mine + t] = {e, at + t * a.tile_rows, min(count - t * a.tile_rows, a.tile_rows), 0};
-      slots += __shfl_sync(0xffffffffu, slot_sum, 31);
-      tiles += __shfl_sync(0xffffffffu, tile_sum, 31);
-    }
-    if (lane == 0) *a.tile_count = tiles;
-  }
+  if (threadIdx.x < 32) lay_out_experts(a, counts, first, lane);
   __syncthreads();
   // (the order of an expert's slots is whatever the counters make it: every slot is computed by itself)
   for (int base = threadIdx.x; base < n; base += U * threads) {
@@ -308,7 +314,7 @@ __global__ void __launch_bounds__(FUSED ? 256 : 1024) route(RouteArgs a) {
         if (lane == 0) a.logits[size_t(row) * logits + e] = sum;
       }
     if (!arrives_last(a.count + 1 + blockIdx.y, gridDim.x, &last)) return;
-    if (warp < rows) choose(a, row0 + warp, lane, ranks[warp], correction);
+    if (warp < rows) choose<false>(a, row0 + warp, lane, ranks[warp], correction);
     if (gridDim.y == 1) __syncthreads();
     else if (!arrives_last(a.count, gridDim.y, &last)) return;
   } else {
@@ -316,10 +322,52 @@ __global__ void __launch_bounds__(FUSED ? 256 : 1024) route(RouteArgs a) {
     allow_dependents();
     const int row = blockIdx.x * warps + warp;
     if (correction) __syncthreads();
-    if (row < a.rows) choose(a, row, lane, ranks[warp], correction);
+    if (row < a.rows) choose<true>(a, row, lane, ranks[warp], correction);
     if (!arrives_last(a.count, gridDim.x, &last)) return;
   }
+  if constexpr (!FUSED) {
+    if (a.rank) {
+      // (every assignment knows its place among its expert's: what is left is where an expert's begin; counts are zero again afterwards)
+      for (int e = threadIdx.x; e < a.experts; e += blockDim.x) {
+        counts[e] = __ldcg(a.tally + e);
+        a.tally[e] = 0;
+      }
+      __syncthreads();
+      if (threadIdx.x < 32) lay_out_experts(a, counts, a.tally + kMaxExperts, lane);
+      return;
+    }
+  }
   sort_assignments(a, counts, first);
+}
+
+// A warp a row: the row to the slots of its assignments, which are entered in the table of slots on the way. A row is read once, in
+// pieces of 128 bytes a lane. (Sorted by one CTA first and gathered by a CTA a slot, 2048 rows of 2048 columns with eight experts each
+// took 34 + 45 us for routing and gathering, now 18 + 32; 67 MB are written.)
+__global__ void __launch_bounds__(256) scatter_rows(RouteArgs a, uint4* out) {
+  dependency_wait();
+  allow_dependents();
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, pieces = a.k_stride / 8;
+  if (row >= a.rows) return;
+  int slot = 0;
+  if (lane < a.top) {
+    const int i = row * a.top + lane;
+    slot = a.tally[kMaxExperts + a.choice[i]] + a.rank[i];
+    a.list[slot] = i;
+    a.slot_score[slot] = a.score[i];
+  }
+  const uint4* from = static_cast<const uint4*>(a.h) + size_t(row) * pieces;
+  for (int at = lane; at - lane < pieces; at += 8 * 32) {      // (the warp stays together: slots are shuffled)
+    uint4 held[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (at + 32 * i < pieces) held[i] = from[at + 32 * i];
+    for (int k = 0; k < a.top; ++k) {
+      uint4* to = out + size_t(__shfl_sync(0xffffffffu, slot, k)) * pieces;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (at + 32 * i < pieces) to[at + 32 * i] = held[i];
+    }
+  }
 }
 
 // out[slot] = h[list[slot] / top], 16 bytes a thread.
@@ -344,9 +392,14 @@ bool RouteFused(int rows) { return rows <= kFusedRows; }
 int Route(const Queue& q, const RouteArgs& a) {
   if (a.rows <= 0) return 0;
   if (a.experts > kMaxExperts || a.top > a.experts || a.top > kMaxTop || a.tile_rows < 1 || a.k_stride % 8 ||
-      (!a.ranks && (a.softmax || a.correction || a.keep_groups < a.groups)) || (a.chosen && a.ranks))
+      (!a.ranks && (a.softmax || a.correction || a.keep_groups < a.groups)) || (a.chosen && a.ranks) || (a.rank && (RouteFused(a.rows) || !a.tally)))
     return int(cudaErrorInvalidValue);
   return q.f32 ? RouteAs<float>(q, a) : RouteAs<__nv_bfloat16>(q, a);
+}
+
+int ScatterRows(const Queue& q, const RouteArgs& a, void* out) {
+  if (q.f32 || !a.rank) return int(cudaErrorInvalidValue);
+  return int(Launch(scatter_rows, dim3(unsigned((a.rows + 7) / 8)), dim3(256), 0, q.stream, q.chained, a, static_cast<uint4*>(out)));
 }
 
 int GatherRows(const Queue& q, const void* h, int k_stride, const ExpertSlots& slots, void* out) {

@@ -232,10 +232,15 @@ struct RouteArgs {
   ExpertTile* tiles;
   int* tile_count;
   unsigned* count;           // kRouteCounters arrival counters, zero between launches
+  // (more rows than RouteFused:) with `rank` the assignments are not sorted; list and slot_score are left to ScatterRows
+  int* rank;                 // [rows * top], place among the expert's assignments
+  int* tally;                // [2 * kMaxExperts]: assignments, zero between launches; first slot
 };
 constexpr int kRouteCounters = 9;
 bool RouteFused(int rows);
 int Route(const Queue& q, const RouteArgs& a);
+// Behind Route with `rank`: list and slot_score, and out[slot] = h[list[slot] / top] (bf16 rows of k_stride).
+int ScatterRows(const Queue& q, const RouteArgs& a, void* out);
 // out[slot] = h[list[slot] / top] (bf16 rows of k_stride).
 int GatherRows(const Queue& q, const void* h, int k_stride, const ExpertSlots& slots, void* out);
 

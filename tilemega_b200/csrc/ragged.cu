@@ -47,6 +47,7 @@ struct RaggedPlan {
   float *score = nullptr, *slot_score = nullptr;
   ExpertTile* tiles = nullptr;
   unsigned* route_count = nullptr;
+  int *rank = nullptr, *tally = nullptr;
   void* gathered = nullptr;        // bf16 plans: [max_rows * most experts of a token][padded width]
   float* ranks = nullptr;          // [max_rows][most experts]
   void* expert_pairs = nullptr;    // fp32 plans: gate/up rows of experts before the gated unit
@@ -534,10 +535,15 @@ int Enqueue(RaggedPlan* plan, uint32_t entries, uint32_t rows, uint32_t longest,
       a.tiles = plan->tiles;
       a.tile_count = plan->tile_count;
       a.count = plan->route_count;
+      const bool gathered = !s.f32 && slots.tile_rows > kGatherRows;
+      if (gathered && !RouteFused(r.rows)) {
+        a.rank = plan->rank;
+        a.tally = plan->tally;
+      }
       if (!RouteFused(r.rows))
         TMB_TRY(Linear(q, linear(plan->normed, layer.router, -1, maps ? &maps->router : nullptr, mlp.logits(), W, plan->logits, mlp.logits(), kLinearFloat)));
       TMB_TRY(Route(q, a));
-      if (!s.f32 && slots.tile_rows > kGatherRows) TMB_TRY(GatherRows(q, plan->normed, W8, slots, plan->gathered));
+      if (gathered) TMB_TRY(a.rank ? ScatterRows(q, a, plan->gathered) : GatherRows(q, plan->normed, W8, slots, plan->gathered));
       const int stride = padded_columns(mlp.ff);
       const Glu glu{float(mlp.limit), float(mlp.alpha), float(mlp.shift), false};
       LinearArgs up = linear(plan->normed, layer.expert_up, -1, maps ? &maps->gate_up : nullptr, mlp.ff, W, plan->expert_hidden, stride, kLinearExpertUp);
@@ -709,6 +715,7 @@ RaggedPlan* RaggedCreate(const RaggedSpec& spec, const std::vector<void*>& buffe
       !Own(plan, &plan->list, slots * sizeof(int)) || !Own(plan, &plan->tile_count, sizeof(int)) ||
       !Own(plan, &plan->score, slots * sizeof(float)) || !Own(plan, &plan->slot_score, slots * sizeof(float)) ||
       !Own(plan, &plan->tiles, (slots / 16 + experts) * sizeof(ExpertTile)) || !Own(plan, &plan->route_count, kRouteCounters * sizeof(unsigned)) ||
+      !Own(plan, &plan->rank, slots * sizeof(int)) || !Own(plan, &plan->tally, top ? 2 * kMaxExperts * sizeof(int) : 0) ||
       !Own(plan, &plan->gathered, spec.f32 ? 0 : slots * W8 * element) ||
       !Own(plan, &plan->expert_hidden, slots * expert_columns * element) || !Own(plan, &plan->expert_out, slots * size_t(spec.width) * element) ||
       !Own(plan, &plan->raw, rows * raw * sizeof(float)) || !Own(plan, &plan->split, spec.f32 ? 0 : rows * split * 2) ||
