@@ -25,6 +25,7 @@
 #include "ptx.cuh"
 #include "tensor_map.h"
 #include "umma.cuh"
+#include "wide.cuh"
 
 namespace tmb {
 namespace {
@@ -296,89 +297,90 @@ __global__ void __launch_bounds__(kGemmThreads, 1) encoder_wide(const __grid_con
   tcgen05_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
+  const int first = blockIdx.x, step = gridDim.x;
   if (warp == 0) {
     if (lane == 0) {
-      int c = 0, issued = 0;
-      bool ok = true, waited = false;
-      for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
-        const int n0 = i / token_tiles * BN, m0 = i % token_tiles * kTileM;
-        const CUtensorMap* wmap = map_of(n0);
-        auto weights = [&](int chunk, int s) {
-          mbar_expect_tx(&full[s], Shape::kStageBytes);
-          tma_load_2d(stages + s * Shape::kStageBytes + kABytes, wmap, chunk * kTileK, n0 % g.n_per_map, &full[s]);
-        };
-        int early = 0;
-        if (!waited) {                       // weights do not depend on the kernel before this one
-          for (; early < S && early < g.kchunks; ++early) weights(early, early);
-          dependency_wait();
-          waited = true;
-        }
-        for (int chunk = 0; chunk < g.kchunks; ++chunk, ++c) {
-          const int s = c % S;
-          if (c >= S) ok = wait_bounded(&empty[s], uint32_t((c / S) - 1) & 1u, g.status, 1);
-          if (!ok) break;
-          if (c >= early) weights(chunk, s);
-          tma_load_2d(stages + s * Shape::kStageBytes, &amap, chunk * kTileK, m0, &full[s]);
-          issued = c + 1;
-        }
-      }
-      if (!ok)   // leaving early: first let the copies already issued land in this CTA's shared memory
-        for (int j = issued > S ? issued - S : 0; j < issued; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
+      int n0 = 0, m0 = 0;
+      const CUtensorMap* wmap = nullptr;
+      const Filled filled = fill_stages<S>(
+          first, step, tiles, g.kchunks,
+          [&](int i) {
+            n0 = i / token_tiles * BN;
+            m0 = i % token_tiles * kTileM;
+            wmap = map_of(n0);
+          },
+          [&](int chunk, int s) {
+            mbar_expect_tx(&full[s], Shape::kStageBytes);
+            tma_load_2d(stages + s * Shape::kStageBytes + kABytes, wmap, chunk * kTileK, n0 % g.n_per_map, &full[s]);
+          },
+          [] { dependency_wait(); }, [&](int chunk, int s) { tma_load_2d(stages + s * Shape::kStageBytes, &amap, chunk * kTileK, m0, &full[s]); },
+          [&](int s, uint32_t parity) { return wait_bounded(&empty[s], parity, g.status, 1); });
+      if (!filled.ok)   // leaving early: first let the copies already issued land in this CTA's shared memory
+        for (int j = filled.chunks > S ? filled.chunks - S : 0; j < filled.chunks; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
     }
   } else if (warp == 1) {
     // the warp walks along together, one lane issues
     const uint32_t idesc = (1u << 4) | Num<T>::kIdescFormat | (uint32_t(BN >> 3) << 17) | (uint32_t(kTileM >> 4) << 24);
     const uint64_t desc = umma_desc_k_sw128(smem_u32(stages), 1024);
     const uint32_t low = uint32_t(desc), high = uint32_t(desc >> 32);
-    int c = 0, k = 0;
-    bool ok = true;
-    for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x, ++k) {
-      if (k > 1) ok = __all_sync(0xffffffffu, wait_bounded(&sum_empty[k & 1], uint32_t((k >> 1) - 1) & 1u, g.status, 3));
-      if (!ok) break;
-      for (int chunk = 0; chunk < g.kchunks; ++chunk, ++c) {
-        const int s = c % S;
-        ok = __all_sync(0xffffffffu, wait_bounded(&full[s], uint32_t(c / S) & 1u, g.status, 3));
-        if (!ok) break;
-        tcgen05_fence_after();
-        if (elect_one()) {
-          const uint32_t a = low + s * (Shape::kStageBytes / 16), b = a + kABytes / 16;
+    uint32_t sum = tmem;
+    multiply_tiles<S>(
+        first, step, tiles, g.kchunks, [&](int, int k) { sum = tmem + (k & 1) * A; },
+        [&](int b, uint32_t parity) {
+          const bool ok = __all_sync(0xffffffffu, wait_bounded(&sum_empty[b], parity, g.status, 3));
+          tcgen05_fence_after();
+          return ok;
+        },
+        [&](int s, uint32_t parity) { return __all_sync(0xffffffffu, wait_bounded(&full[s], parity, g.status, 3)) != 0; },
+        [&](int chunk, int s) {
+          tcgen05_fence_after();
+          if (elect_one()) {
+            const uint32_t a = low + s * (Shape::kStageBytes / 16), b = a + kABytes / 16;
 #pragma unroll
-          for (int j = 0; j < kTileK / 16; ++j) umma_step(tmem + (k & 1) * A, a + 2 * j, b + 2 * j, high, idesc, (chunk | j) != 0);
-          umma_commit(&empty[s]);
-        }
-        __syncwarp();
-      }
-      if (elect_one()) umma_commit(&sum_full[k & 1]);
-      __syncwarp();
-    }
-    if (!ok)
-      for (int j = 0; j < 1000000 && !mbar_try_wait(&sum_full[k & 1], uint32_t(k >> 1) & 1u); ++j) {
-      }
+            for (int j = 0; j < kTileK / 16; ++j) umma_step(sum, a + 2 * j, b + 2 * j, high, idesc, (chunk | j) != 0);
+            umma_commit(&empty[s]);
+          }
+          __syncwarp();
+        },
+        [&](int b) {
+          if (elect_one()) umma_commit(&sum_full[b]);
+          __syncwarp();
+        },
+        [&](int b, uint32_t parity) {
+          for (int j = 0; j < 1000000 && !mbar_try_wait(&sum_full[b], parity); ++j) {
+          }
+        });
   } else {
     const int quarter = warp & 3, column_half = (warp - 2) >> 2;
-    int k = 0;
-    for (int i = blockIdx.x; i < tiles; i += gridDim.x, ++k) {
-      const int n0 = i / token_tiles * BN, row = i % token_tiles * kTileM + 32 * quarter + lane;
-      if (EPI != kEpiPartial) {              // the tile's bias (weights: no need to wait for the kernel before)
-        const int e = threadIdx.x - 64;
-        if (e < BN / 8)
-          reinterpret_cast<uint4*>(bias_tile[k & 1])[e] =
-              __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(g.bias[n0 / g.n_per_map]) + n0 % g.n_per_map) + e);
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-      }
-      if (k == 0) dependency_wait();
-      if (!__all_sync(0xffffffffu, wait_bounded(&sum_full[k & 1], uint32_t(k >> 1) & 1u, g.status, 4))) break;
-      tcgen05_fence_after();
-      if (i + int(gridDim.x) >= tiles) allow_dependents();
+    write_tiles(
+        first, step, tiles,
+        [&](int i, int k) {
+          if (EPI != kEpiPartial) {            // the tile's bias (weights: no need to wait for the kernel before)
+            const int n0 = i / token_tiles * BN, e = threadIdx.x - 64;
+            if (e < BN / 8)
+              reinterpret_cast<uint4*>(bias_tile[k & 1])[e] =
+                  __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(g.bias[n0 / g.n_per_map]) + n0 % g.n_per_map) + e);
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+          }
+          if (k == 0) dependency_wait();
+        },
+        [&](int b, uint32_t parity) {
+          const bool ok = __all_sync(0xffffffffu, wait_bounded(&sum_full[b], parity, g.status, 4));
+          tcgen05_fence_after();
+          return ok;
+        },
+        [&](int i, int k, bool last) {
+          if (last) allow_dependents();
+          const int n0 = i / token_tiles * BN, row = i % token_tiles * kTileM + 32 * quarter + lane;
 #pragma unroll 1
-      for (int c = column_half * (BN / 2); c < (column_half + 1) * (BN / 2); c += 32) {
-        float v[32];
-        tmem_load_32(tmem + (k & 1) * A + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
-        write_columns<T, EPI, 32>(v, static_cast<T*>(g.out), reinterpret_cast<float*>(g.out), size_t(row) * g.ldc + n0 + c, bias_tile[k & 1], c);
-      }
-      tcgen05_fence_before();
-      mbar_arrive(&sum_empty[k & 1]);
-    }
+          for (int c = column_half * (BN / 2); c < (column_half + 1) * (BN / 2); c += 32) {
+            float v[32];
+            tmem_load_32(tmem + (k & 1) * A + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
+            write_columns<T, EPI, 32>(v, static_cast<T*>(g.out), reinterpret_cast<float*>(g.out), size_t(row) * g.ldc + n0 + c, bias_tile[k & 1], c);
+          }
+          tcgen05_fence_before();
+        },
+        [&](int b) { mbar_arrive(&sum_empty[b]); });
   }
   tcgen05_fence_before();
   __syncthreads();

@@ -1,0 +1,80 @@
+// The roles of a persistent product (encoder_wide): a CTA takes every `step`-th tile from `first` on. One warp fills a ring of S
+// stages with the chunks of K of tile after tile, one issues the products into one of two accumulators, eight warps write the other
+// one out. Everything that touches memory or a barrier is the caller's (a wait returns false once it has given up), so that
+// the roles also run on the host, against waits that fail there.
+#pragma once
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define TMB_ROLE __device__ __forceinline__
+#else
+#define TMB_ROLE inline
+#endif
+
+namespace tmb {
+
+struct Filled {
+  int chunks;      // requested
+  bool ok;
+};
+
+// tile(i): the tile from here on; weights(chunk, s), rows(chunk, s): copies of one chunk; inputs_there(): before the first rows.
+template <int S, class Tile, class Weights, class There, class Rows, class Empty>
+TMB_ROLE Filled fill_stages(int first, int step, int tiles, int chunks, Tile tile, Weights weights, There inputs_there, Rows rows, Empty empty) {
+  int c = 0;
+  bool ok = true;
+  for (int i = first; i < tiles && ok; i += step) {
+    tile(i);
+    int early = 0;
+    if (i == first) {                     // weights do not depend on the kernel before this one
+      for (; early < S && early < chunks; ++early) weights(early, early);
+      inputs_there();
+    }
+    for (int chunk = 0; chunk < chunks; ++chunk, ++c) {
+      const int s = c % S;
+      if (c >= S) ok = empty(s, uint32_t(c / S - 1) & 1u);
+      if (!ok) break;
+      if (c >= early) weights(chunk, s);
+      rows(chunk, s);
+    }
+  }
+  return {c, ok};
+}
+
+// tile(i, k): the CTA's k-th tile from here on; products(chunk, s): of one chunk, behind them the stage is free;
+// commit(b): sum_full[b] arrives once all products so far are done; done(b, parity): waits for that.
+template <int S, class Tile, class SumEmpty, class Full, class Products, class Commit, class Done>
+TMB_ROLE void multiply_tiles(int first, int step, int tiles, int chunks, Tile tile, SumEmpty sum_empty, Full full, Products products, Commit commit, Done done) {
+  int c = 0, k = 0;
+  bool ok = true;
+  for (int i = first; i < tiles && ok; i += step, ++k) {
+    if (k > 1) ok = sum_empty(k & 1, uint32_t((k >> 1) - 1) & 1u);
+    if (!ok) break;
+    tile(i, k);
+    for (int chunk = 0; chunk < chunks; ++chunk, ++c) {
+      const int s = c % S;
+      ok = full(s, uint32_t(c / S) & 1u);
+      if (!ok) break;
+      products(chunk, s);
+    }
+    commit(k & 1);
+  }
+  if (!ok) done(k & 1, uint32_t(k >> 1) & 1u);
+}
+
+// begin(i, k): before the wait for the CTA's k-th tile, where the warps may meet: all of them come there for every tile, also behind a
+// wait that gave up in one of them. write(i, k, last) puts the tile out; written(k & 1) gives its accumulator back.
+template <class Begin, class SumFull, class Write, class Written>
+TMB_ROLE void write_tiles(int first, int step, int tiles, Begin begin, SumFull sum_full, Write write, Written written) {
+  bool ok = true;
+  int k = 0;
+  for (int i = first; i < tiles; i += step, ++k) {
+    begin(i, k);
+    ok = ok && sum_full(k & 1, uint32_t(k >> 1) & 1u);
+    if (!ok) continue;
+    write(i, k, i + step >= tiles);
+    written(k & 1);
+  }
+}
+
+}  // namespace tmb
