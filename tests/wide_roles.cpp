@@ -1,7 +1,8 @@
 // The roles of a persistent product (tilemega_b200/csrc/wide.cuh) on host threads, with barriers, copies and products that behave as
 // the device's do: copies land in any order, products run one after the other behind their issue. A CTA by itself, and a pair whose
-// first CTA issues for both. Every wait of every role is made to give up once; a role that never ends, a product on a stage that does
-// not hold its chunk, or a tile written from sums that are not its own ends the program with a message.
+// first CTA issues for both. Every wait of every role is made to give up once; a role that never ends, a product that is still under
+// way where tensor memory is freed, a product on a stage that does not hold its chunk, or a tile written from sums that are not its
+// own ends the program with a message.
 #include <unistd.h>
 
 #include <condition_variable>
@@ -190,7 +191,8 @@ struct Cta {
         },
         [&](int b, uint32_t parity) {
           std::unique_lock<std::mutex> lock(sim.m);
-          sim.changed.wait_for(lock, std::chrono::milliseconds(20), [&] { return sum_full[b].complete(parity); });
+          if (!sim.changed.wait_for(lock, std::chrono::seconds(2), [&] { return sum_full[b].complete(parity); }))
+            fail("a wait for products that nobody commits", sim.fail_role, sim.fail_wait);
         });
   }
   void write(int warp) {
@@ -239,6 +241,7 @@ bool attempt(bool pair, int role, int wait, unsigned seed) {
   if (pair) other->start(roles);
   for (auto& thread : roles) thread.join();
   std::lock_guard<std::mutex> lock(sim.m);
+  if (sim.products) fail("products under way where tensor memory is freed", role, wait);
   if (sim.failed) return true;
   one.each([&](Cta& cta) {
     for (int i = 1; i < kTiles; i += kStep)

@@ -346,10 +346,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) encoder_wide(const __grid_con
           if (elect_one()) umma_commit(&sum_full[b]);
           __syncwarp();
         },
-        [&](int b, uint32_t parity) {
-          for (int j = 0; j < 1000000 && !mbar_try_wait(&sum_full[b], parity); ++j) {
-          }
-        });
+        [&](int b, uint32_t parity) { drained(&sum_full[b], parity); });
   } else {
     const int quarter = warp & 3, column_half = (warp - 2) >> 2;
     write_tiles(

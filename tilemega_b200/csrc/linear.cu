@@ -15,6 +15,7 @@
 #include "ptx.cuh"
 #include "tensor_map.h"
 #include "umma.cuh"
+#include "wide.cuh"
 
 namespace tmb {
 namespace {
@@ -451,151 +452,151 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
     if (lane == 0) {
       constexpr int kBoxes = PerExpert(EPI) ? kWide / 32 : 1;      // (per expert by 32 rows: only those there cost anything)
       constexpr int kBoxBytes = Shape::kTokens / kBoxes * kStepK * 2;
-      int c = 0, issued = 0;                          // chunks so far
-      bool ok = true, waited = false;
+      WideTile tile;
+      int boxes = 1;
       auto load = [&](unsigned char* to, const CUtensorMap* map, int x, int y, int s) {
         if constexpr (PAIR) tma_load_2d_pair(to, map, x, y, &full[s]);
         else tma_load_2d(to, map, x, y, &full[s]);
       };
-      auto weights = [&](const WideTile& tile, int chunk, int s, int boxes) {
-        if (rank == 0) mbar_expect_tx(&full[s], uint32_t(kCtas * (kWeightBytes + boxes * kBoxBytes)));
-        load(stages + s * Shape::kStageBytes, &wmap, chunk * kStepK, tile.weight_row, s);
-      };
-      for (int i = first; i < tiles && ok; i += step) {
-        const WideTile tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
-        const int boxes = PerExpert(EPI) ? (tile.t_end - tile.t0 + 31) / 32 : 1, row0 = tile.t0 + int(rank) * Shape::kTokens;
-        int early = 0;
-        if (!waited) {                                // weights do not depend on the kernel before this one
-          for (; early < min(S, g.chunks); ++early) weights(tile, early, early, boxes);
-          dependency_wait();
-          waited = true;
-        }
-        for (int chunk = 0; chunk < g.chunks; ++chunk, ++c) {
-          const int s = c % S;
-          if (c >= S) ok = wait_bounded(&empty[s], uint32_t((c / S) - 1) & 1u, g.status, 1);
-          if (!ok) break;
-          if (c >= early) weights(tile, chunk, s, boxes);
-          unsigned char* rows = stages + s * Shape::kStageBytes + kWeightBytes;
-          for (int j = 0; j < boxes; ++j) load(rows + j * kBoxBytes, &tmap, tile.k_at + chunk * kStepK, row0 + j * (Shape::kTokens / kBoxes), s);
-          issued = c + 1;
-        }
-      }
-      if (!ok && rank == 0)   // leaving early: let the copies already issued land first
-        for (int j = issued > S ? issued - S : 0; j < issued; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
+      const Filled filled = fill_stages<S>(
+          first, step, tiles, g.chunks,
+          [&](int i) {
+            tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
+            if (PerExpert(EPI)) boxes = (tile.t_end - tile.t0 + 31) / 32;
+          },
+          [&](int chunk, int s) {
+            if (rank == 0) mbar_expect_tx(&full[s], uint32_t(kCtas * (kWeightBytes + boxes * kBoxBytes)));
+            load(stages + s * Shape::kStageBytes, &wmap, chunk * kStepK, tile.weight_row, s);
+          },
+          [] { dependency_wait(); },
+          [&](int chunk, int s) {
+            unsigned char* rows = stages + s * Shape::kStageBytes + kWeightBytes;
+            for (int j = 0; j < boxes; ++j)
+              load(rows + j * kBoxBytes, &tmap, tile.k_at + chunk * kStepK, tile.t0 + int(rank) * Shape::kTokens + j * (Shape::kTokens / kBoxes), s);
+          },
+          [&](int s, uint32_t parity) { return wait_bounded(&empty[s], parity, g.status, 1); });
+      if (!filled.ok && rank == 0)   // leaving early: let the copies already issued land first
+        for (int j = filled.chunks > S ? filled.chunks - S : 0; j < filled.chunks; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
     }
   } else if (warp == 1) {
-    // the warp walks along together, one lane issues
+    // the warp walks along together, one lane issues (of a pair the first CTA's)
     const uint64_t desc = umma_desc_k_sw128(smem_u32(stages), 1024);
     const uint32_t low = uint32_t(desc), high = uint32_t(desc >> 32);
-    int c = 0, k = 0;
-    bool ok = true;
-    for (int i = first; i < tiles && ok && rank == 0; i += step, ++k) {
-      const int columns = PerExpert(EPI) ? __shfl_sync(0xffffffffu, wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there).columns, 0) : kWide;
-      const uint32_t idesc = umma_idesc_bf16(kCtas * kRowsM, columns), sum = tmem + (k & 1) * kWide;
-      if (k > 1) ok = __all_sync(0xffffffffu, wait_bounded(&sum_empty[k & 1], uint32_t((k >> 1) - 1) & 1u, g.status, 3));
-      if (!ok) break;
-      tcgen05_fence_after();
-      for (int chunk = 0; chunk < g.chunks; ++chunk, ++c) {
-        const int s = c % S;
-        ok = __all_sync(0xffffffffu, wait_bounded(&full[s], uint32_t(c / S) & 1u, g.status, 3));
-        if (!ok) break;
-        tcgen05_fence_after();
-        if (elect_one()) {
-          const uint32_t w = low + s * (Shape::kStageBytes / 16), t = w + kWeightBytes / 16;
+    uint32_t idesc = umma_idesc_bf16(kCtas * kRowsM, kWide), sum = tmem;
+    multiply_tiles<S>(
+        first, step, rank == 0 ? tiles : 0, g.chunks,
+        [&](int i, int k) {
+          if (PerExpert(EPI)) idesc = umma_idesc_bf16(kRowsM, __shfl_sync(0xffffffffu, wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there).columns, 0));
+          sum = tmem + (k & 1) * kWide;
+        },
+        [&](int b, uint32_t parity) {
+          const bool ok = __all_sync(0xffffffffu, wait_bounded(&sum_empty[b], parity, g.status, 3));
+          tcgen05_fence_after();
+          return ok;
+        },
+        [&](int s, uint32_t parity) { return __all_sync(0xffffffffu, wait_bounded(&full[s], parity, g.status, 3)) != 0; },
+        [&](int chunk, int s) {
+          tcgen05_fence_after();
+          if (elect_one()) {
+            const uint32_t w = low + s * (Shape::kStageBytes / 16), t = w + kWeightBytes / 16;
 #pragma unroll
-          for (int j = 0; j < kStepK / 16; ++j) {
-            if constexpr (PAIR) umma_step_pair(sum, w + 2 * j, t + 2 * j, high, idesc, (chunk | j) != 0);
-            else umma_step(sum, w + 2 * j, t + 2 * j, high, idesc, (chunk | j) != 0);
+            for (int j = 0; j < kStepK / 16; ++j) {
+              if constexpr (PAIR) umma_step_pair(sum, w + 2 * j, t + 2 * j, high, idesc, (chunk | j) != 0);
+              else umma_step(sum, w + 2 * j, t + 2 * j, high, idesc, (chunk | j) != 0);
+            }
+            if constexpr (PAIR) umma_commit_pair(&empty[s]);
+            else umma_commit(&empty[s]);
           }
-          if constexpr (PAIR) umma_commit_pair(&empty[s]);
-          else umma_commit(&empty[s]);
-        }
-        __syncwarp();
-      }
-      if (elect_one()) {                              // arrives once everything issued above is done
-        if constexpr (PAIR) umma_commit_pair(&sum_full[k & 1]);
-        else umma_commit(&sum_full[k & 1]);
-      }
-      __syncwarp();
-    }
-    if (!ok)
-      for (int j = 0; j < 1000000 && !mbar_try_wait(&sum_full[k & 1], uint32_t(k >> 1) & 1u); ++j) {
-      }
+          __syncwarp();
+        },
+        [&](int b) {
+          if (elect_one()) {                            // arrives once everything issued above is done
+            if constexpr (PAIR) umma_commit_pair(&sum_full[b]);
+            else umma_commit(&sum_full[b]);
+          }
+          __syncwarp();
+        },
+        [&](int b, uint32_t parity) { drained(&sum_full[b], parity); });
   } else {
     const int quarter = warp & 3, column_half = (warp - 2) >> 2;
-    bool ok = true, waited = false;
-    int k = 0;
-    for (int i = first; i < tiles; i += step, ++k) {
-      const WideTile tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
-      const int n0 = tile.n0, t0 = tile.t0, t_end = tile.t_end, out_at = tile.out_at;
-      if (!waited) dependency_wait();
-      waited = true;
-      ok = __all_sync(0xffffffffu, wait_bounded(&sum_full[k & 1], uint32_t(k >> 1) & 1u, g.status, 4));
-      if (!ok) break;
-      tcgen05_fence_after();
-      if (i + step >= tiles) allow_dependents();
-      const uint32_t sum = tmem + (k & 1) * kWide;
-      const int n = n0 + 32 * quarter + lane;
-      const float bias = g.bias && n < g.n ? g.bias[n] : 0.f;
-      for (int c = column_half * (kWide / 2); c < (column_half + 1) * (kWide / 2); c += 32) {
-        if (t0 + c >= t_end) break;
-        float v[32];
-        tmem_load_32(sum + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
-        const int cols = min(32, t_end - t0 - c);
-        if constexpr (IsGlu(EPI)) {
-          const bool upper = lane >= kGluUnit;          // lanes 0..15 hold gate rows, 16..31 the matching up rows
-          const int out = (n0 + 32 * quarter) / 2 + (lane & (kGluUnit - 1));
+    write_tiles(
+        first, step, tiles,
+        [&](int, int k) {
+          if (k == 0) dependency_wait();
+        },
+        [&](int b, uint32_t parity) {
+          const bool ok = __all_sync(0xffffffffu, wait_bounded(&sum_full[b], parity, g.status, 4));
+          tcgen05_fence_after();
+          return ok;
+        },
+        [&](int i, int k, bool last) {
+          if (last) allow_dependents();
+          const WideTile tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
+          const int n0 = tile.n0, t0 = tile.t0, t_end = tile.t_end, out_at = tile.out_at;
+          const uint32_t sum = tmem + (k & 1) * kWide;
+          const int n = n0 + 32 * quarter + lane;
+          const float bias = g.bias && n < g.n ? g.bias[n] : 0.f;
+          for (int c = column_half * (kWide / 2); c < (column_half + 1) * (kWide / 2); c += 32) {
+            if (t0 + c >= t_end) break;
+            float v[32];
+            tmem_load_32(sum + (uint32_t(32 * quarter) << 16) + uint32_t(c), v);
+            const int cols = min(32, t_end - t0 - c);
+            if constexpr (IsGlu(EPI)) {
+              const bool upper = lane >= kGluUnit;          // lanes 0..15 hold gate rows, 16..31 the matching up rows
+              const int out = (n0 + 32 * quarter) / 2 + (lane & (kGluUnit - 1));
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {             // lower lanes finish column i, upper lanes column i + 1
-            const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + 1], kGluUnit);
-            const float y = glu_value(upper ? other : v[i], upper ? v[i + 1] : other, g.glu);
-            const int col = i + (upper ? 1 : 0);
-            if (out < g.outputs && col < cols)
-              static_cast<__nv_bfloat16*>(g.out)[size_t(t0 + c + col) * g.out_stride + out] = __float2bfloat16_rn(y);
-          }
-        } else if constexpr (EPI == kLinearRotate) {
-          const Turn turn = turn_of(g.rotate, n);
-          if (__any_sync(0xffffffffu, turn.on)) {
+              for (int i = 0; i < 32; i += 2) {             // lower lanes finish column i, upper lanes column i + 1
+                const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + 1], kGluUnit);
+                const float y = glu_value(upper ? other : v[i], upper ? v[i + 1] : other, g.glu);
+                const int col = i + (upper ? 1 : 0);
+                if (out < g.outputs && col < cols)
+                  static_cast<__nv_bfloat16*>(g.out)[size_t(t0 + c + col) * g.out_stride + out] = __float2bfloat16_rn(y);
+              }
+            } else if constexpr (EPI == kLinearRotate) {
+              const Turn turn = turn_of(g.rotate, n);
+              if (__any_sync(0xffffffffu, turn.on)) {
 #pragma unroll
-            for (int i0 = 0; i0 < 32; i0 += 8) {
-              float2 angle[8];
+                for (int i0 = 0; i0 < 32; i0 += 8) {
+                  float2 angle[8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) angle[i] = angle_at(g.rotate, turn, t0 + c + min(i0 + i, cols - 1));
+                  for (int i = 0; i < 8; ++i) angle[i] = angle_at(g.rotate, turn, t0 + c + min(i0 + i, cols - 1));
 #pragma unroll
-              for (int i = 0; i < 8; ++i) v[i0 + i] = turned(turn, angle[i], v[i0 + i], __shfl_xor_sync(0xffffffffu, v[i0 + i], 1));
+                  for (int i = 0; i < 8; ++i) v[i0 + i] = turned(turn, angle[i], v[i0 + i], __shfl_xor_sync(0xffffffffu, v[i0 + i], 1));
+                }
+              }
+              if (n < g.n) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (i < cols) emit<EPI>(g, t0 + c + i, n, v[i]);
+              }
+            } else if (n < g.n) {
+              if constexpr (EPI == kLinearAdd) {
+                float* x = static_cast<float*>(g.out) + size_t(t0 + c) * g.out_stride + n;
+                float old[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (i < cols) old[i] = x[size_t(i) * g.out_stride];
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (i < cols) x[size_t(i) * g.out_stride] = old[i] + (v[i] + bias);
+              } else {
+                if (EPI == kLinearStore && n0 < g.tanh_below) {
+#pragma unroll
+                  for (int i = 0; i < 32; ++i)
+                    if (n < g.tanh_below) v[i] = tanh16(v[i] + bias) - bias;
+                }
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (i < cols) emit<EPI>(g, t0 + c + i, out_at + n, v[i] + bias);
+              }
             }
           }
-          if (n < g.n) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < cols) emit<EPI>(g, t0 + c + i, n, v[i]);
-          }
-        } else if (n < g.n) {
-          if constexpr (EPI == kLinearAdd) {
-            float* x = static_cast<float*>(g.out) + size_t(t0 + c) * g.out_stride + n;
-            float old[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < cols) old[i] = x[size_t(i) * g.out_stride];
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < cols) x[size_t(i) * g.out_stride] = old[i] + (v[i] + bias);
-          } else {
-            if (EPI == kLinearStore && n0 < g.tanh_below) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (n < g.tanh_below) v[i] = tanh16(v[i] + bias) - bias;
-            }
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < cols) emit<EPI>(g, t0 + c + i, out_at + n, v[i] + bias);
-          }
-        }
-      }
-      tcgen05_fence_before();
-      if constexpr (PAIR) arrive_at(&sum_empty[k & 1], 0);
-      else mbar_arrive(&sum_empty[k & 1]);
-    }
+          tcgen05_fence_before();
+        },
+        [&](int b) {
+          if constexpr (PAIR) arrive_at(&sum_empty[b], 0);
+          else mbar_arrive(&sum_empty[b]);
+        });
   }
   tcgen05_fence_before();
   __syncthreads();

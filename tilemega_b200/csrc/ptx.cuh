@@ -330,6 +330,15 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, uns
   return true;
 }
 
+// Wait for what this CTA has under way before it leaves, also behind a wait that gave up: only time ends it.
+constexpr unsigned long long kDrainLimitNs = 100000000ull;
+__device__ __forceinline__ bool drained(uint64_t* bar, uint32_t parity) {
+  const unsigned long long start = global_timer();
+  while (!mbar_try_wait(bar, parity))
+    if (global_timer() - start > kDrainLimitNs) return false;
+  return true;
+}
+
 // 32 consecutive fp32 columns of this thread's tensor-memory lane in one instruction.
 __device__ __forceinline__ void tmem_load_32(uint32_t address, float (&v)[32]) {
   uint32_t r[32];

@@ -1,4 +1,4 @@
-// The roles of a persistent product (encoder_wide): a CTA takes every `step`-th tile from `first` on. One warp fills a ring of S
+// The roles of a persistent product (linear_wide, encoder_wide): a CTA, or a pair of them, takes every `step`-th tile from `first` on. One warp fills a ring of S
 // stages with the chunks of K of tile after tile, one issues the products into one of two accumulators, eight warps write the other
 // one out. Everything that touches memory or a barrier is the caller's (a wait returns false once it has given up), so that
 // the roles also run on the host, against waits that fail there.
@@ -42,10 +42,11 @@ TMB_ROLE Filled fill_stages(int first, int step, int tiles, int chunks, Tile til
 }
 
 // tile(i, k): the CTA's k-th tile from here on; products(chunk, s): of one chunk, behind them the stage is free;
-// commit(b): sum_full[b] arrives once all products so far are done; done(b, parity): waits for that.
+// commit(b): sum_full[b] arrives once all products so far are done; done(b, parity): waits for that, for a limited time. The role ends behind
+// the last commit's arrival, whatever the writers do: no product is under way any more when tensor memory goes.
 template <int S, class Tile, class SumEmpty, class Full, class Products, class Commit, class Done>
 TMB_ROLE void multiply_tiles(int first, int step, int tiles, int chunks, Tile tile, SumEmpty sum_empty, Full full, Products products, Commit commit, Done done) {
-  int c = 0, k = 0;
+  int c = 0, k = 0, last = -1;        // last: the tile committed last
   bool ok = true;
   for (int i = first; i < tiles && ok; i += step, ++k) {
     if (k > 1) ok = sum_empty(k & 1, uint32_t((k >> 1) - 1) & 1u);
@@ -58,8 +59,9 @@ TMB_ROLE void multiply_tiles(int first, int step, int tiles, int chunks, Tile ti
       products(chunk, s);
     }
     commit(k & 1);
+    last = k;
   }
-  if (!ok) done(k & 1, uint32_t(k >> 1) & 1u);
+  if (last >= 0) done(last & 1, uint32_t(last >> 1) & 1u);
 }
 
 // begin(i, k): before the wait for the CTA's k-th tile, where the warps may meet: all of them come there for every tile, also behind a
