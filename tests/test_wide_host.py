@@ -1,5 +1,5 @@
 """The roles of the persistent products (tilemega_b200/csrc/wide.cuh) on host threads: tiles, stages and accumulators take their turns, and
-whichever wait gives up, every role ends, behind the last product."""
+whichever wait gives up, every role ends, behind the last product and copy."""
 import shutil
 import subprocess
 from pathlib import Path

@@ -1,7 +1,7 @@
 // The roles of a persistent product (tilemega_b200/csrc/wide.cuh) on host threads, with barriers, copies and products that behave as
 // the device's do: copies land in any order, products run one after the other behind their issue. A CTA by itself, and a pair whose
-// first CTA issues for both. Every wait of every role is made to give up once; a role that never ends, a product that is still under
-// way where tensor memory is freed, a product on a stage that does not hold its chunk, or a tile written from sums that are not its
+// first CTA issues for both. Every wait of every role is made to give up once; a role that never ends, a product or a copy that is
+// still under way where the CTAs go, a product on a stage that does not hold its chunk, or a tile written from sums that are not its
 // own ends the program with a message.
 #include <unistd.h>
 
@@ -131,6 +131,11 @@ struct Cta {
     f(*first);
     if (first->second) f(*first->second);
   }
+  void landed(int s, uint32_t parity) {
+    std::unique_lock<std::mutex> lock(sim.m);
+    if (!sim.changed.wait_for(lock, std::chrono::seconds(2), [&] { return full[s].complete(parity); }))
+      fail("copies that never count as landed", sim.fail_role, sim.fail_wait);
+  }
   void load() {
     int tile = -1, waits = 0;
     bool there = false;
@@ -158,6 +163,18 @@ struct Cta {
           copy(&rows[s], chunk, s);
         },
         [&](int s, uint32_t parity) { return sim.wait(empty[s], parity, role(0), waits); });
+    if (shares() == 1 && !filled.ok) tmb::drain_stages<S>(filled.chunks, [&](int s, uint32_t parity) { landed(s, parity); });
+  }
+  // (of a pair's first CTA, behind the end of both)
+  void drain() {
+    if (filled.ok && second->filled.ok) return;
+    auto at = [&](int s, auto what) {
+      std::lock_guard<std::mutex> lock(sim.m);
+      what(full[s]);
+    };
+    tmb::drain_pair<S>(
+        filled.chunks, second->filled.chunks, [&](int s) { at(s, [](Sim::Bar& bar) { bar.landed(2 * kBytes); }); },
+        [&](int s) { at(s, [](Sim::Bar& bar) { bar.arrive(2 * kBytes); }); }, [&](int s, uint32_t parity) { landed(s, parity); });
   }
   void multiply() {
     int waits = 0, tile = -1, sum = 0;
@@ -240,8 +257,10 @@ bool attempt(bool pair, int role, int wait, unsigned seed) {
   one.start(roles);
   if (pair) other->start(roles);
   for (auto& thread : roles) thread.join();
+  if (pair) one.drain();
   std::lock_guard<std::mutex> lock(sim.m);
   if (sim.products) fail("products under way where tensor memory is freed", role, wait);
+  if (sim.copies) fail("copies under way where the CTAs go", role, wait);
   if (sim.failed) return true;
   one.each([&](Cta& cta) {
     for (int i = 1; i < kTiles; i += kStep)

@@ -315,8 +315,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) encoder_wide(const __grid_con
           },
           [] { dependency_wait(); }, [&](int chunk, int s) { tma_load_2d(stages + s * Shape::kStageBytes, &amap, chunk * kTileK, m0, &full[s]); },
           [&](int s, uint32_t parity) { return wait_bounded(&empty[s], parity, g.status, 1); });
-      if (!filled.ok)   // leaving early: first let the copies already issued land in this CTA's shared memory
-        for (int j = filled.chunks > S ? filled.chunks - S : 0; j < filled.chunks; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
+      if (!filled.ok) drain_stages<S>(filled.chunks, [&](int s, uint32_t parity) { drained(&full[s], parity); });
     }
   } else if (warp == 1) {
     // the warp walks along together, one lane issues

@@ -419,9 +419,11 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t full[S], empty[S], sum_full[2], sum_empty[2];     // (pairs: full and sum_empty are the first CTA's)
   __shared__ uint32_t tmem_slot;
+  __shared__ int progress[2];                                           // (pairs) chunks that each CTA requested, n for ok or -1 - n
   unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_rank() : 0;
+  auto landed = [&](int s, uint32_t parity) { drained(&full[s], parity); };
   // (tables of tiles and counts of rows were written before the kernel in front of this one, see linear_tiles)
   int t_there = g.t;
   if (EPI == kLinearStore && g.rows_there) t_there = min(t_there, *g.rows_there);
@@ -475,8 +477,12 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
               load(rows + j * kBoxBytes, &tmap, tile.k_at + chunk * kStepK, tile.t0 + int(rank) * Shape::kTokens + j * (Shape::kTokens / kBoxes), s);
           },
           [&](int s, uint32_t parity) { return wait_bounded(&empty[s], parity, g.status, 1); });
-      if (!filled.ok && rank == 0)   // leaving early: let the copies already issued land first
-        for (int j = filled.chunks > S ? filled.chunks - S : 0; j < filled.chunks; ++j) wait_bounded(&full[j % S], uint32_t(j / S) & 1u, g.status, 2);
+      if constexpr (PAIR) {
+        progress[rank] = filled.ok ? filled.chunks : -1 - filled.chunks;
+        store_at(&progress[rank], rank ^ 1u, progress[rank]);
+      } else if (!filled.ok) {
+        drain_stages<S>(filled.chunks, landed);
+      }
     }
   } else if (warp == 1) {
     // the warp walks along together, one lane issues (of a pair the first CTA's)
@@ -600,7 +606,17 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
   }
   tcgen05_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync();                  // (neither is gone while the other still signals it)
+  if constexpr (PAIR) {
+    cluster_sync();                                      // (neither is gone while the other still signals it)
+    if (progress[0] < 0 || progress[1] < 0) {            // a wait gave up: what either loader requested lands before both go
+      constexpr uint32_t kShare = Shape::kStageBytes;    // a CTA's bytes of a chunk
+      auto count = [&](int of) { return progress[of] < 0 ? -1 - progress[of] : progress[of]; };
+      if (rank == 0 && threadIdx.x == 0)
+        drain_pair<S>(
+            count(0), count(1), [&](int s) { mbar_complete_tx(&full[s], kShare); }, [&](int s) { mbar_expect_tx(&full[s], kShare); }, landed);
+      cluster_sync();
+    }
+  }
   if (warp == 1) {
     tcgen05_fence_after();
     if constexpr (PAIR) tmem_dealloc_pair(tmem, 512);

@@ -62,6 +62,9 @@ __device__ __forceinline__ uint32_t address_in(const void* local, uint32_t rank)
 __device__ __forceinline__ void arrive_at(uint64_t* bar, uint32_t rank) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(address_in(bar, rank)) : "memory");
 }
+__device__ __forceinline__ void store_at(int* local, uint32_t rank, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(address_in(local, rank)), "r"(v) : "memory");
+}
 // As tma_load_2d into this CTA's memory, counted on the first CTA's barrier.
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tensor_map, int x, int y, uint64_t* bar) {
   asm volatile(

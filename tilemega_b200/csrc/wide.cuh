@@ -15,10 +15,11 @@ namespace tmb {
 
 struct Filled {
   int chunks;      // requested
-  bool ok;
+  bool ok;         // and multiplied: no copy is under way any more, nor an arrival on one of this CTA's barriers
 };
 
 // tile(i): the tile from here on; weights(chunk, s), rows(chunk, s): copies of one chunk; inputs_there(): before the first rows.
+// Not ok: the copies of the last S chunks may be under way still (drain_stages, drain_pair).
 template <int S, class Tile, class Weights, class There, class Rows, class Empty>
 TMB_ROLE Filled fill_stages(int first, int step, int tiles, int chunks, Tile tile, Weights weights, There inputs_there, Rows rows, Empty empty) {
   int c = 0;
@@ -38,7 +39,25 @@ TMB_ROLE Filled fill_stages(int first, int step, int tiles, int chunks, Tile til
       rows(chunk, s);
     }
   }
+  for (int j = c > S ? c - S : 0; j < c && ok; ++j) ok = empty(j % S, uint32_t(j / S) & 1u);
   return {c, ok};
+}
+
+// Before the CTA may go: landed(s, parity) waits for a phase of full[s], for a limited time.
+template <int S, class Landed> TMB_ROLE void drain_stages(int chunks, Landed landed) {
+  for (int j = chunks > S ? chunks - S : 0; j < chunks; ++j) landed(j % S, uint32_t(j / S) & 1u);
+}
+// The same for a pair whose copies all count on the first CTA's barriers, by the first CTA, once both loaders have ended: they may have
+// requested different numbers of chunks. without(s): the second CTA's share of a chunk will not come; only(s): nothing but that will.
+template <int S, class Without, class Only, class Landed> TMB_ROLE void drain_pair(int mine, int peers, Without without, Only only, Landed landed) {
+  const int both = mine < peers ? mine : peers, all = mine < peers ? peers : mine;
+  for (int j = all > S ? all - S : 0; j < all; ++j) {
+    if (j >= both) {
+      if (mine > peers) without(j % S);
+      else only(j % S);
+    }
+    landed(j % S, uint32_t(j / S) & 1u);
+  }
 }
 
 // tile(i, k): the CTA's k-th tile from here on; products(chunk, s): of one chunk, behind them the stage is free;
