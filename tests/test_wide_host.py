@@ -1,4 +1,4 @@
-"""The roles of the persistent products (tilemega_b200/csrc/wide.cuh) on host threads: tiles, stages and accumulators take their turns, and
+"""The roles of the persistent products and of the loader of portions' keys (tilemega_b200/csrc/wide.cuh) on host threads: tiles, stages and accumulators take their turns, and
 whichever wait gives up, every role ends, behind the last product and copy."""
 import shutil
 import subprocess

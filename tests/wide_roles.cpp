@@ -1,8 +1,8 @@
-// The roles of a persistent product (tilemega_b200/csrc/wide.cuh) on host threads, with barriers, copies and products that behave as
-// the device's do: copies land in any order, products run one after the other behind their issue. A CTA by itself, and a pair whose
-// first CTA issues for both. Every wait of every role is made to give up once; a role that never ends, a product or a copy that is
-// still under way where the CTAs go, a product on a stage that does not hold its chunk, or a tile written from sums that are not its
-// own ends the program with a message.
+// The roles of tilemega_b200/csrc/wide.cuh (persistent products; the loader of portions' keys and values) on host threads, with
+// barriers, copies and products that behave as the device's do: copies land in any order, products run one after the other behind
+// their issue. A CTA by itself, and a pair whose first CTA issues for both; blocks of keys and values, some halves not full. Every wait
+// of every role is made to give up once; a role that never ends, a product or a copy that is still under way where the CTAs go, a
+// product on a stage that does not hold its chunk, or a tile written from sums that are not its own ends the program with a message.
 #include <unistd.h>
 
 #include <condition_variable>
@@ -247,7 +247,96 @@ struct Cta {
   }
 };
 
+// Keys and values: role 0 loads, role 1 stands for the products that read them.
+struct Blocks {
+  static constexpr int KS = 2, VS = 3;
+  Sim& sim;
+  int count;
+  bool ragged;             // the last block is not full
+  Sim::Bar k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], v_landed;
+  Sim::Stage keys[KS], values[VS];
+  int seen = 0;
+
+  Blocks(Sim& s, int n, bool r) : sim(s), count(n), ragged(r) {}
+  bool is_part(int b, int half) const { return ragged && (b == count - 1 || (b == 1 && half == 1)); }
+  void copy(Sim::Stage* stage, Sim::Stage is, Sim::Bar* bar) {
+    bar->arrive(kBytes);
+    ++sim.copies;
+    sim.copying.push_back([=, this] {
+      *stage = is;
+      bar->landed(kBytes);
+      --sim.copies;
+    });
+    sim.changed.notify_all();
+  }
+  void load() {
+    int waits = 0, moved = -1;
+    auto drained = [&](Sim::Bar& bar, uint32_t parity) {
+      std::unique_lock<std::mutex> lock(sim.m);
+      if (!sim.changed.wait_for(lock, std::chrono::seconds(2), [&] { return bar.complete(parity); }))
+        fail("copies that never count as landed", sim.fail_role, sim.fail_wait);
+    };
+    tmb::fill_blocks<KS, VS>(
+        count,
+        [&](int b, int s) {
+          std::lock_guard<std::mutex> lock(sim.m);
+          copy(&keys[s], {b, 0}, &k_full[s]);
+        },
+        [&](int b, int half, int s) {
+          std::lock_guard<std::mutex> lock(sim.m);
+          if (b != moved) fail("values of another block", 0, waits);
+          copy(&values[s], {b, half}, is_part(b, half) ? &v_landed : &v_full[s]);
+          return is_part(b, half);
+        },
+        [&](uint32_t parity) { return sim.wait(v_landed, parity, 0, waits); },
+        [&](int b, int half, int s) {
+          std::lock_guard<std::mutex> lock(sim.m);
+          if (values[s].tile != b || values[s].chunk != half) fail("a half that has not landed", sim.fail_role, sim.fail_wait);
+          v_full[s].arrive();
+          sim.changed.notify_all();
+        },
+        [&](int b) { moved = b + 1; }, [&](int s, uint32_t parity) { return sim.wait(k_empty[s], parity, 0, waits); },
+        [&](int s, uint32_t parity) { return sim.wait(v_empty[s], parity, 0, waits); }, [&](int s, uint32_t parity) { drained(k_full[s], parity); },
+        [&](int s, uint32_t parity) { drained(v_full[s], parity); }, [&](uint32_t parity) { drained(v_landed, parity); });
+  }
+  void read() {
+    int waits = 0;
+    auto product = [&](Sim::Stage* held, Sim::Stage is, Sim::Bar* empty) {
+      std::lock_guard<std::mutex> lock(sim.m);
+      sim.queue.push_back([=, this] {
+        if (held->tile != is.tile || held->chunk != is.chunk) fail("a product on another block's stage", sim.fail_role, sim.fail_wait);
+        empty->arrive();
+        ++seen;
+      });
+      sim.changed.notify_all();
+    };
+    for (int b = 0; b <= count; ++b) {
+      if (b < count) {
+        if (!sim.wait(k_full[b % KS], uint32_t(b / KS) & 1u, 1, waits)) return;
+        product(&keys[b % KS], {b, 0}, &k_empty[b % KS]);
+      }
+      for (int v = 2 * b - 2; b > 0 && v < 2 * b; ++v) {
+        if (!sim.wait(v_full[v % VS], uint32_t(v / VS) & 1u, 1, waits)) return;
+        product(&values[v % VS], {b - 1, v & 1}, &v_empty[v % VS]);
+      }
+    }
+  }
+};
+
 // One run; false: its failing wait was never reached.
+bool attempt_blocks(int count, int role, int wait, unsigned seed) {
+  Sim sim(role, wait, seed);
+  Blocks blocks(sim, count, count % 2);
+  std::thread load([&] { blocks.load(); }), read([&] { blocks.read(); });
+  load.join();
+  read.join();
+  std::unique_lock<std::mutex> lock(sim.m);
+  if (sim.copies) fail("copies under way where the CTA goes", role, wait);
+  sim.changed.wait(lock, [&] { return sim.queue.empty(); });
+  if (!sim.failed && blocks.seen != 3 * count) fail("a block not read", role, wait);
+  return sim.failed;
+}
+
 bool attempt(bool pair, int role, int wait, unsigned seed) {
   Sim sim(role, wait, seed);
   Cta one(sim, nullptr);
@@ -275,13 +364,19 @@ bool attempt(bool pair, int role, int wait, unsigned seed) {
 int main() {
   alarm(90);               // (a role that never ends)
   int runs = 0;
-  for (unsigned seed = 0; seed < 6; ++seed)
+  for (unsigned seed = 0; seed < 6; ++seed) {
+    for (int count : {1, 2, 6, 7}) {
+      if (attempt_blocks(count, -1, 0, seed)) return 1;
+      for (int role : {0, 1})
+        for (int wait = 0; attempt_blocks(count, role, wait, seed * 1000 + unsigned(wait)); ++wait) ++runs;
+    }
     for (bool pair : {false, true}) {
       if (attempt(pair, -1, 0, seed)) return 1;
       for (int role : {0, 1, 2, 5, 9, 20, 22, 26})
         if (pair || role < 20)
           for (int wait = 0; attempt(pair, role, wait, seed * 1000 + unsigned(wait)); ++wait) ++runs;
     }
+  }
   std::printf("%d waits gave up, every role ended\n", runs);
   return 0;
 }

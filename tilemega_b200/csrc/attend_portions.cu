@@ -5,6 +5,7 @@
 #include "attend.cuh"
 #include "tensor_map.h"
 #include "umma.cuh"
+#include "wide.cuh"
 
 namespace tmb {
 namespace {
@@ -160,7 +161,6 @@ __global__ void __launch_bounds__(PortionShape<KC, VC, TILES>::kThreads, 1) atte
         if (p.context) return context + j;
         return key_row(table, j, r) / kRun * p.kv_heads + group;
       };
-      bool ok = true;
       // up to `most` runs of a block from its run `first` on, as `chunks` pieces of 64 columns
       auto issue = [&](const CUtensorMap* map, unsigned char* to, int chunks, int chunk_bytes, uint64_t* full, int b, int first, int most, int at) {
         const int runs = min(max((block_limit(b) - block_base(b) + kRun - 1) / kRun - first, 0), most);
@@ -170,41 +170,33 @@ __global__ void __launch_bounds__(PortionShape<KC, VC, TILES>::kThreads, 1) atte
         if (run >= 0 && run < runs)
           for (int c = 0; c < chunks; ++c) tma_load_3d(to + c * chunk_bytes + run * kRun * 128, map, 64 * c, p.context ? group : 0, at, full);
       };
-      int at_value = 0, at_key = place(0), at_next = blocks > 1 ? place(1) : 0, keys = 0, values = 0, parts = 0;
-      for (int b = -1; b < blocks && ok; ++b) {        // keys of block b + 1, values of block b; places are fetched one turn ahead
-        if (b + 1 < blocks) {
-          const int stage = (b + 1) % KS, turn = (b + 1) / KS;
-          if (turn > 0) ok = __all_sync(0xffffffffu, wait_bounded(&k_empty[stage], (turn - 1) & 1, status, kWaitLoader));
-          if (!ok) break;
-          issue(&k_map, ks + stage * KC * kChunk, KC, kChunk, &k_full[stage], b + 1, 0, kRuns, at_key);
-          ++keys;
-        }
-        for (int half = 0; half < 2 && b >= 0; ++half) {
-          const int stage = (2 * b + half) % VS, turn = (2 * b + half) / VS, there = max(0, block_limit(b) - block_base(b) - half * kHalfKeys);
-          if (turn > 0) ok = __all_sync(0xffffffffu, wait_bounded(&v_empty[stage], (turn - 1) & 1, status, kWaitLoader));
-          if (!ok) break;
-          unsigned char* to = vs + stage * VC * kHalfChunk;
-          const bool part = there < kHalfKeys;
-          issue(&v_map, to, VC, kHalfChunk, part ? &v_landed : &v_full[stage], b, half * kRuns / 2, kRuns / 2, at_value);
-          if (part) {                                  // what lies behind the last key, or was there before, may be no number
-            ok = __all_sync(0xffffffffu, wait_bounded(&v_landed, parts++ & 1, status, kWaitLoader));
-            if (!ok) break;
-            for (int i = lane; i < (kHalfKeys - there) * 8 * VC; i += 32)
-              *reinterpret_cast<uint4*>(to + (i / 8 % VC) * kHalfChunk + (there + i / (8 * VC)) * 128 + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+      auto there = [&](int b, int half) { return max(0, block_limit(b) - block_base(b) - half * kHalfKeys); };      // values of a half
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_bounded(bar, parity, status, kWaitLoader)) != 0; };
+      int at_value = 0, at_key = place(0), at_next = blocks > 1 ? place(1) : 0;      // places are fetched one turn ahead
+      fill_blocks<KS, VS>(
+          blocks, [&](int b, int s) { issue(&k_map, ks + s * KC * kChunk, KC, kChunk, &k_full[s], b, 0, kRuns, at_key); },
+          [&](int b, int half, int s) {
+            const bool part = there(b, half) < kHalfKeys;
+            issue(&v_map, vs + s * VC * kHalfChunk, VC, kHalfChunk, part ? &v_landed : &v_full[s], b, half * kRuns / 2, kRuns / 2, at_value);
+            return part;
+          },
+          [&](uint32_t parity) { return wait(&v_landed, parity); },
+          [&](int b, int half, int s) {                // what lies behind the last key, or was there before, may be no number
+            const int held = there(b, half);
+            for (int i = lane; i < (kHalfKeys - held) * 8 * VC; i += 32)
+              *reinterpret_cast<uint4*>(vs + s * VC * kHalfChunk + (i / 8 % VC) * kHalfChunk + (held + i / (8 * VC)) * 128 + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&v_full[stage]);
-          }
-          ++values;
-        }
-        at_value = at_key;
-        at_key = at_next;
-        at_next = b + 3 < blocks ? place(b + 3) : 0;
-      }
-      if (!ok) {                                       // leaving early: let the copies already issued land first
-        for (int b = max(0, keys - KS); b < keys; ++b) wait_bounded(&k_full[b % KS], (b / KS) & 1, status, kWaitLoader);
-        for (int i = max(0, values - VS); i < values; ++i) wait_bounded(&v_full[i % VS], (i / VS) & 1, status, kWaitLoader);
-      }
+            if (lane == 0) mbar_arrive(&v_full[s]);
+          },
+          [&](int b) {
+            at_value = at_key;
+            at_key = at_next;
+            at_next = b + 3 < blocks ? place(b + 3) : 0;
+          },
+          [&](int s, uint32_t parity) { return wait(&k_empty[s], parity); }, [&](int s, uint32_t parity) { return wait(&v_empty[s], parity); },
+          [&](int s, uint32_t parity) { drained(&k_full[s], parity); }, [&](int s, uint32_t parity) { drained(&v_full[s], parity); },
+          [&](uint32_t parity) { drained(&v_landed, parity); });
     } else if (warp == 4 * TILES) {
       // ---- products: the warp walks along together, one lane issues (what decides its way is taken from votes and shuffles, so that
       // the compiler knows it to be the warp's: operands of the products are then formed once, not per lane) ----
@@ -268,9 +260,7 @@ __global__ void __launch_bounds__(PortionShape<KC, VC, TILES>::kThreads, 1) atte
         for (int t = 0; t < TILES; ++t) umma_commit(&o_full[t]);
       __syncwarp();
       // (also behind a wait that gave up: tensor memory is freed once no product runs)
-      for (int t = 0; t < TILES; ++t)
-        for (int i = 0; i < 1000000 && !mbar_try_wait(&o_full[t], 0); ++i) {
-        }
+      for (int t = 0; t < TILES; ++t) drained(&o_full[t], 0);
     }
   } else {
     if constexpr (TILES == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");

@@ -1,7 +1,7 @@
 // The roles of a persistent product (linear_wide, encoder_wide): a CTA, or a pair of them, takes every `step`-th tile from `first` on. One warp fills a ring of S
 // stages with the chunks of K of tile after tile, one issues the products into one of two accumulators, eight warps write the other
 // one out. Everything that touches memory or a barrier is the caller's (a wait returns false once it has given up), so that
-// the roles also run on the host, against waits that fail there.
+// the roles also run on the host, against waits that fail there. Below them the loader of attend_portions, for the same reason.
 #pragma once
 #include <stdint.h>
 
@@ -96,6 +96,46 @@ TMB_ROLE void write_tiles(int first, int step, int tiles, Begin begin, SumFull s
     write(i, k, i + step >= tiles);
     written(k & 1);
   }
+}
+
+// Blocks of keys and values for attend_portions, through rings of KS whole blocks of keys and VS half blocks of values; the keys of a
+// block are requested before the values of the one before it. keys(b, s), values(b, half, s): copies; the latter is true for a half
+// that is not full, whose copies count on a barrier of their own, part_landed(parity), before part(b, half, s) hands it on.
+// moved(b): places of later blocks. A wait that gave up: the *_drained wait for what was requested, for a limited time.
+template <int KS, int VS, class Keys, class Values, class PartLanded, class Part, class Moved, class KeyEmpty, class ValueEmpty, class KeyDrained, class ValueDrained,
+          class PartDrained>
+TMB_ROLE bool fill_blocks(int blocks, Keys keys, Values values, PartLanded part_landed, Part part, Moved moved, KeyEmpty key_empty, ValueEmpty value_empty,
+                          KeyDrained key_drained, ValueDrained value_drained, PartDrained part_drained) {
+  int k = 0, v = 0, parts = 0;
+  bool ok = true, landing = false;
+  for (int b = -1; b < blocks && ok; ++b) {
+    if (b + 1 < blocks) {
+      if (k >= KS) ok = key_empty(k % KS, uint32_t(k / KS - 1) & 1u);
+      if (!ok) break;
+      keys(b + 1, k % KS);
+      ++k;
+    }
+    for (int half = 0; half < 2 && b >= 0; ++half) {
+      if (v >= VS) ok = value_empty(v % VS, uint32_t(v / VS - 1) & 1u);
+      if (!ok) break;
+      if (values(b, half, v % VS)) {
+        ok = part_landed(uint32_t(parts) & 1u);
+        landing = !ok;
+        if (!ok) break;
+        part(b, half, v % VS);
+        ++parts;
+      }
+      ++v;
+    }
+    moved(b);
+  }
+  for (int j = k > KS ? k - KS : 0; j < k && ok; ++j) ok = key_empty(j % KS, uint32_t(j / KS) & 1u);
+  for (int j = v > VS ? v - VS : 0; j < v && ok; ++j) ok = value_empty(j % VS, uint32_t(j / VS) & 1u);
+  if (ok) return true;
+  for (int j = k > KS ? k - KS : 0; j < k; ++j) key_drained(j % KS, uint32_t(j / KS) & 1u);
+  for (int j = v > VS ? v - VS : 0; j < v; ++j) value_drained(j % VS, uint32_t(j / VS) & 1u);
+  if (landing) part_drained(uint32_t(parts) & 1u);
+  return false;
 }
 
 }  // namespace tmb
