@@ -6,6 +6,7 @@ import bamudra_case
 import benarax_case
 import nadilorn_case
 from test_gpu_ragged import executor, run_cut
+from tilemega_b200.serving.ragged import Portion
 
 pytestmark = pytest.mark.gpu
 
@@ -38,6 +39,36 @@ def test_rotation(plan_dir):
     case = benarax_case
     config = case.model(96, 131, [case.latent(60, 120, 40, 40, 130, 72), case.latent(60, 96, 64, 24, 260, 40, neighbours=False)], groups=2, taps=3)
     check(case, config, case.weights_for(config, "bf16"), plan_dir, ([512, 18], [300, 230]))
+
+
+def test_products_by_heads(plan_dir):
+    """Latent attention whose latent rows are small enough that portions are not expanded: every row's queries and values pass through
+    products by heads, of 128 rows a head, 200 and 48. And one of 308 rows a head, where only a decoded token beside the portion does."""
+    case = benarax_case
+    config = case.model(96, 131, [case.latent(64, 64, 8, 128, 40, 24), case.latent(32, 56, 8, 200, 40, 24, neighbours=False), case.latent(24, 40, 8, 72, 300, 24)],
+                        groups=2)
+    tensors = case.weights_for(config, "bf16")
+    check(case, config, tensors, plan_dir, ([512, 18], [300, 230]))
+    single, portion = case.tokens(config, 41, seed=3), case.tokens(config, 530, seed=4)
+    with executor(config, tensors, plan_dir, "bf16", capacity=640, max_rows=640, max_wanted=640) as ex:
+        slots = ex.open(), ex.open()
+        ex.run([Portion(slots[0], single[:40])])
+        logits = ex.run([Portion(slots[0], single[40:], [0]), Portion(slots[1], portion, list(range(530)))])
+    assert case.error(logits[:1], case.truth(config, tensors, single)[0][40:]) < case.TOLERANCE["bf16"]
+    assert case.error(logits[1:], case.truth(config, tensors, portion)[0]) < case.TOLERANCE["bf16"]
+
+
+def test_pairs_that_would_take_a_round_more(plan_dir):
+    """49 tiles of weight rows by three of tokens: single CTAs, for the gated unit and the head, a stream's sums, and rotated queries."""
+    case = nadilorn_case
+    config = case.model(96, 6272, [case.layer(4, 2, 32, 32, 16, 90, case.dense(3136))])
+    check(case, config, case.weights(config), plan_dir, ([530],))
+    case = bamudra_case
+    config = case.model(6272, 131, [case.attention_layer(4, 2, 64, 32, 100, 3, mlp=case.mlp(80, 1.5))])
+    check(case, config, case.weights(config), plan_dir, ([530],))
+    case = benarax_case
+    config = case.model(96, 131, [case.latent(56, 80, 32, 40, 130, 72)], groups=2)
+    check(case, config, case.weights_for(config, "bf16"), plan_dir, ([530],))
 
 
 @pytest.mark.parametrize("module", [nadilorn_case, benarax_case], ids=["input weighted", "output weighted"])

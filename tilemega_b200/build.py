@@ -38,7 +38,7 @@ UNIT_HEADERS = {"megakernel.cu": KERNEL_HEADERS, "static_probe.cu": KERNEL_HEADE
                 "plan_spec.cpp": SPEC_HEADERS, "runtime.cu": SPEC_HEADERS + ("encoder.h", "ragged.h"),
                 "encoder.cu": SPEC_HEADERS + ("encoder.h", "ptx.cuh", "tensor_map.h", "umma.cuh", "wide.cuh"), "absent.cu": SPEC_HEADERS + ("encoder.h",),
                 "ragged_spec.cpp": SPEC_HEADERS + ("ragged_limits.h",), "ragged.cu": SPEC_HEADERS + OP_HEADERS + ("ragged.h",),
-                "linear.cu": OP_HEADERS + ("umma.cuh", "wide.cuh"), "rows.cu": OP_HEADERS, "experts.cu": OP_HEADERS, "mixers.cu": OP_HEADERS + ("mixers.cuh",),
+                "linear.cu": OP_HEADERS + ("umma.cuh", "wide.cuh", "linear_rules.h"), "rows.cu": OP_HEADERS, "experts.cu": OP_HEADERS, "mixers.cu": OP_HEADERS + ("mixers.cuh",),
                 "mixers_mma.cu": OP_HEADERS + ("mixers.cuh", "mma.cuh", "attend.cuh"), "attend_portions.cu": OP_HEADERS + ("mixers.cuh", "mma.cuh", "attend.cuh", "umma.cuh", "wide.cuh"),
                 "latent.cu": OP_HEADERS + ("mixers.cuh", "mma.cuh"),
                 "delta.cu": OP_HEADERS + ("mixers.cuh",), "delta_mma.cu": OP_HEADERS + ("mixers.cuh", "mma.cuh"), "conv.cu": OP_HEADERS}

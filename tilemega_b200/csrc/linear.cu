@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "element.cuh"
+#include "linear_rules.h"
 #include "ops.h"
 #include "ptx.cuh"
 #include "tensor_map.h"
@@ -20,11 +21,9 @@
 namespace tmb {
 namespace {
 
-constexpr int kRowsM = 128;                 // weight rows per tile
 constexpr int kStepK = 64;                  // 16-bit elements per 128-byte swizzle row
 constexpr int kWeightBytes = kRowsM * kStepK * 2;
 constexpr int kLinearThreads = 320;         // producer warp, issuing warp, eight epilogue warps
-constexpr int kMaxCluster = 8;
 
 struct LinearParams {
   const float* bias;
@@ -365,14 +364,13 @@ __global__ void __launch_bounds__(kLinearThreads) linear_tiles(const __grid_cons
 // products, and the copies never stop between tiles. Tiles are counted tokens first, per expert weight rows first, as in
 // linear_tiles.
 //
-// PAIR (all but experts): the two CTAs of a cluster work on 256 weight rows x 256 tokens together. Each brings its own 128 weight rows
+// PAIR (ChooseLinear): the two CTAs of a cluster work on 256 weight rows x 256 tokens together. Each brings its own 128 weight rows
 // and 128 of the tokens, the first issues the products of both, and each has the sums of its weight rows. A chunk of K then costs a CTA
 // 32 KB instead of 48, which is what L2 can deliver at the tensor pipe's pace. Bound by the tensor pipe and by the last round of tiles
 // (256 tiles over 74 pairs are four rounds for three and a half). 2048 tokens, width 4096: gated unit of 28672 rows 321 us (1.50 PFLOP/s, 0.91
 // of the measured cuBLAS rate) where single tiles of a CTA each took 431; projection of 10240 rows 120 for 150; outputs of K 4096 and 14336
 // 121 for 133 on average. Experts: 128 of 1152 x 2048 with some 128 rows each 164 and 147 us for 169 and 190 (their weights alone are 94 us of
 // copying), because an expert of 129 to 256 rows now reads its weights once.
-constexpr int kWide = 256;
 template <bool PAIR> struct WideShape {
   static constexpr int kTokens = PAIR ? kWide / 2 : kWide;             // whose rows a CTA brings
   static constexpr int kStages = PAIR ? 6 : 4, kStageBytes = kWeightBytes + kTokens * kStepK * 2;
@@ -383,9 +381,10 @@ struct WideTile {
   int n0, t0, t_end, weight_row, k_at, out_at, columns;
 };
 
-template <int EPI> __device__ __forceinline__ WideTile wide_tile(const LinearParams& g, int i, int token_tiles, int weight_tiles, int t_there) {
+template <int EPI, bool PAIR> __device__ __forceinline__ WideTile wide_tile(const LinearParams& g, int i, int token_tiles, int weight_tiles, int t_there) {
   WideTile tile{};
-  constexpr int kRows = PerExpert(EPI) ? kRowsM : 2 * kRowsM;          // weight rows of a tile
+  constexpr int kRows = PAIR ? 2 * kRowsM : kRowsM;                    // weight rows of a tile
+  const int mine = PAIR ? int(cluster_rank()) * kRowsM : 0;            // from which on they are this CTA's
   if constexpr (PerExpert(EPI)) {
     const ExpertTile e = g.slots.tiles[i / weight_tiles];
     tile.n0 = i % weight_tiles * kRowsM;
@@ -397,11 +396,11 @@ template <int EPI> __device__ __forceinline__ WideTile wide_tile(const LinearPar
     const int w = i / token_tiles;
     tile.t0 = i % token_tiles * kWide;
     tile.t_end = t_there;
-    tile.n0 = tile.weight_row = w * kRows + int(cluster_rank()) * kRowsM;
+    tile.n0 = tile.weight_row = w * kRows + mine;
     tile.columns = kWide;
     if constexpr (EPI == kLinearHeads) {
       const int per_head = (g.n + kRows - 1) / kRows, head = w / per_head;
-      tile.n0 = w % per_head * kRows + int(cluster_rank()) * kRowsM;
+      tile.n0 = w % per_head * kRows + mine;
       tile.weight_row = head * g.n + tile.n0;
       tile.k_at = head * g.head_in;
       tile.out_at = head * g.head_out;
@@ -410,10 +409,10 @@ template <int EPI> __device__ __forceinline__ WideTile wide_tile(const LinearPar
   return tile;
 }
 
-template <int EPI>
+template <int EPI, bool PAIR>
 __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap tmap,
                                                                  const LinearParams g, int weight_tiles) {
-  constexpr bool PAIR = !PerExpert(EPI);
+  static_assert(!(PAIR && (PerExpert(EPI) || EPI == kLinearHeads)));
   using Shape = WideShape<PAIR>;
   constexpr int S = Shape::kStages, kCtas = PAIR ? 2 : 1;
   extern __shared__ unsigned char smem_raw[];
@@ -463,7 +462,7 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
       const Filled filled = fill_stages<S>(
           first, step, tiles, g.chunks,
           [&](int i) {
-            tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
+            tile = wide_tile<EPI, PAIR>(g, i, token_tiles, weight_tiles, t_there);
             if (PerExpert(EPI)) boxes = (tile.t_end - tile.t0 + 31) / 32;
           },
           [&](int chunk, int s) {
@@ -492,7 +491,7 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
     multiply_tiles<S>(
         first, step, rank == 0 ? tiles : 0, g.chunks,
         [&](int i, int k) {
-          if (PerExpert(EPI)) idesc = umma_idesc_bf16(kRowsM, __shfl_sync(0xffffffffu, wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there).columns, 0));
+          if (PerExpert(EPI)) idesc = umma_idesc_bf16(kRowsM, __shfl_sync(0xffffffffu, wide_tile<EPI, PAIR>(g, i, token_tiles, weight_tiles, t_there).columns, 0));
           sum = tmem + (k & 1) * kWide;
         },
         [&](int b, uint32_t parity) {
@@ -537,7 +536,7 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
         },
         [&](int i, int k, bool last) {
           if (last) allow_dependents();
-          const WideTile tile = wide_tile<EPI>(g, i, token_tiles, weight_tiles, t_there);
+          const WideTile tile = wide_tile<EPI, PAIR>(g, i, token_tiles, weight_tiles, t_there);
           const int n0 = tile.n0, t0 = tile.t0, t_end = tile.t_end, out_at = tile.out_at;
           const uint32_t sum = tmem + (k & 1) * kWide;
           const int n = n0 + 32 * quarter + lane;
@@ -710,22 +709,34 @@ template <int BN> cudaError_t RaiseLimit() {
   return cudaSuccess;
 }
 
-// Most tiles the slots of a step can fall into: full ones, and one more for every expert in use.
-int MostTiles(const ExpertSlots& s) { return s.slots / s.tile_rows + std::min(s.experts, s.slots); }
+template <bool PAIR> cudaError_t RaiseWide() {
+  for (auto kernel : {linear_wide<kLinearStore, PAIR>, linear_wide<kLinearAdd, PAIR>, linear_wide<kLinearGlu, PAIR>, linear_wide<kLinearFloat, PAIR>,
+                      linear_wide<kLinearRotate, PAIR>, linear_wide<kLinearSide, PAIR>}) {
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<PAIR>::kSmem);
+    if (err != cudaSuccess) return err;
+  }
+  return cudaSuccess;
+}
 
+int MostTiles(const ExpertSlots& s) { return MostExpertTiles(s.slots, s.experts, s.tile_rows); }
+
+template <bool PAIR>
 cudaError_t LaunchWide(const Queue& q, const LinearArgs& a, const LinearParams& p) {
-  auto kernel = a.epilogue == kLinearAdd ? linear_wide<kLinearAdd> : a.epilogue == kLinearGlu ? linear_wide<kLinearGlu>
-                : a.epilogue == kLinearFloat ? linear_wide<kLinearFloat> : a.epilogue == kLinearExpertUp ? linear_wide<kLinearExpertUp>
-                : a.epilogue == kLinearExpertDown ? linear_wide<kLinearExpertDown> : a.epilogue == kLinearHeads ? linear_wide<kLinearHeads>
-                : a.epilogue == kLinearExpertGlu ? linear_wide<kLinearExpertGlu> : a.epilogue == kLinearRotate ? linear_wide<kLinearRotate>
-                : a.epilogue == kLinearSide ? linear_wide<kLinearSide> : linear_wide<kLinearStore>;
-  const bool pair = !PerExpert(a.epilogue);
-  const int rows = pair ? 2 * kRowsM : kRowsM, weight_tiles = (a.n + rows - 1) / rows * std::max(a.heads, 1);
-  const long long tiles = (long long)(weight_tiles) * (pair ? (a.t + kWide - 1) / kWide : MostTiles(a.slots));
+  auto kernel = a.epilogue == kLinearAdd ? linear_wide<kLinearAdd, PAIR> : a.epilogue == kLinearGlu ? linear_wide<kLinearGlu, PAIR>
+                : a.epilogue == kLinearFloat ? linear_wide<kLinearFloat, PAIR> : a.epilogue == kLinearRotate ? linear_wide<kLinearRotate, PAIR>
+                : a.epilogue == kLinearSide ? linear_wide<kLinearSide, PAIR> : linear_wide<kLinearStore, PAIR>;
+  if constexpr (!PAIR) {
+    if (a.epilogue == kLinearHeads) kernel = linear_wide<kLinearHeads, false>;
+    if (a.epilogue == kLinearExpertUp) kernel = linear_wide<kLinearExpertUp, false>;
+    if (a.epilogue == kLinearExpertDown) kernel = linear_wide<kLinearExpertDown, false>;
+    if (a.epilogue == kLinearExpertGlu) kernel = linear_wide<kLinearExpertGlu, false>;
+  }
+  const int rows = PAIR ? 2 * kRowsM : kRowsM, weight_tiles = (a.n + rows - 1) / rows * std::max(a.heads, 1);
+  const long long tiles = (long long)(weight_tiles) * (PerExpert(a.epilogue) ? MostTiles(a.slots) : (a.t + kWide - 1) / kWide);
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(pair ? 2 * unsigned(std::min<long long>(tiles, q.sm_count / 2)) : unsigned(std::min<long long>(tiles, q.sm_count)));
+  config.gridDim = dim3(PAIR ? 2 * unsigned(std::min<long long>(tiles, q.sm_count / 2)) : unsigned(std::min<long long>(tiles, q.sm_count)));
   config.blockDim = dim3(kLinearThreads);
-  config.dynamicSmemBytes = pair ? WideShape<true>::kSmem : WideShape<false>::kSmem;
+  config.dynamicSmemBytes = WideShape<PAIR>::kSmem;
   config.stream = q.stream;
   cudaLaunchAttribute attributes[2];
   int count = 0;
@@ -733,7 +744,7 @@ cudaError_t LaunchWide(const Queue& q, const LinearArgs& a, const LinearParams& 
     attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attributes[count++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (pair) {
+  if (PAIR) {
     attributes[count].id = cudaLaunchAttributeClusterDimension;
     attributes[count].val.clusterDim.x = 2;
     attributes[count].val.clusterDim.y = 1;
@@ -741,7 +752,7 @@ cudaError_t LaunchWide(const Queue& q, const LinearArgs& a, const LinearParams& 
   }
   config.attrs = attributes;
   config.numAttrs = unsigned(count);
-  return cudaLaunchKernelEx(&config, kernel, a.maps->weight, a.maps->rows[pair ? 3 : 1], p, weight_tiles);
+  return cudaLaunchKernelEx(&config, kernel, a.maps->weight, a.maps->rows[PAIR ? 3 : PerExpert(a.epilogue) ? 1 : 4], p, weight_tiles);
 }
 
 template <int BN>
@@ -775,51 +786,18 @@ cudaError_t LaunchTiles(const Queue& q, const LinearArgs& a, const LinearParams&
   return cudaLaunchKernelEx(&config, kernel, a.maps->weight, Gathers(a.epilogue, BN) ? a.maps->row : a.maps->rows[PerExpert(a.epilogue) ? std::min(map, 1) : map], p);
 }
 
-// Tile width (index into 16, 32, 64, 128, 256 tokens) and K splits: the widest tile that gives most SMs a CTA, else
-// the narrowest that covers the tokens (at most 128), with K split over a cluster until the SMs are covered; further, up
-// to two CTAs per SM, where a part keeps a long run of K.
-void ChooseLinear(int t, int n, int heads, int chunks, int sms, int* index, int* splits) {
-  const int tiles = (n + kRowsM - 1) / kRowsM * heads;
-  *splits = 1;
-  if (t > 128 && tiles * ((t + 255) / 256) * 10 >= sms * 8) {
-    *index = 4;
-    return;
-  }
-  *index = 0;
-  while (*index < 3 && (16 << *index) < t) ++*index;
-  const int grid = tiles * ((t + (16 << *index) - 1) / (16 << *index));
-  while (*splits < kMaxCluster && grid * *splits <= sms && chunks / (*splits * 2) >= (grid * *splits * 10 < sms * 8 ? 4 : 16)) *splits *= 2;
-}
-
-// The same per expert: the tile width is that of the slot table; K splits until the tiles to be expected cover the SMs.
-void ChooseExpertLinear(const ExpertSlots& s, int n, int chunks, int sms, int* index, int* splits) {
-  *index = 0;
-  while ((16 << *index) < s.tile_rows) ++*index;
-  *splits = 1;
-  if (*index == 4) return;
-  const int grid = MostTiles(s) * ((n + kRowsM - 1) / kRowsM);
-  while (*splits < kMaxCluster && grid * *splits <= sms && chunks / (*splits * 2) >= 4) *splits *= 2;
-}
-
 }  // namespace
 
-int ExpertTileRows(const Queue& q, int slots, int experts) {
-  if (q.f32) return kTile32;
-  const int share = (slots + experts - 1) / experts;   // slots of an expert on average; most have no more than 4/3 of it
-  int rows = 16;
-  while (rows < kWide && rows * 3 < share * 4) rows *= 2;
-  return rows;
-}
+int ExpertTileRows(const Queue& q, int slots, int experts) { return q.f32 ? kTile32 : ExpertRows(slots, experts); }
 
 int PrepareLinear() {
   cudaError_t err = RaiseLimit<16>();
   if (err == cudaSuccess) err = RaiseLimit<32>();
   if (err == cudaSuccess) err = RaiseLimit<64>();
   if (err == cudaSuccess) err = RaiseLimit<128>();
-  for (auto kernel : {linear_wide<kLinearStore>, linear_wide<kLinearAdd>, linear_wide<kLinearGlu>, linear_wide<kLinearFloat>, linear_wide<kLinearHeads>,
-                      linear_wide<kLinearRotate>, linear_wide<kLinearSide>})
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<true>::kSmem);
-  for (auto kernel : {linear_wide<kLinearExpertUp>, linear_wide<kLinearExpertDown>, linear_wide<kLinearExpertGlu>})
+  if (err == cudaSuccess) err = RaiseWide<true>();
+  if (err == cudaSuccess) err = RaiseWide<false>();
+  for (auto kernel : {linear_wide<kLinearHeads, false>, linear_wide<kLinearExpertUp, false>, linear_wide<kLinearExpertDown, false>, linear_wide<kLinearExpertGlu, false>})
     if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WideShape<false>::kSmem);
   return int(err);
 }
@@ -876,16 +854,15 @@ int Linear(const Queue& q, const LinearArgs& a) {
                       static_cast<const float*>(a.weight), p, a.k_stride, a.in_stride ? a.in_stride : a.k_stride));
   }
   p.chunks = (a.k_stride + kStepK - 1) / kStepK;
-  int index = 0, splits = 1;
-  if (experts) ChooseExpertLinear(a.slots, a.n, p.chunks, q.sm_count, &index, &splits);
-  else ChooseLinear(a.t, a.n, std::max(a.heads, 1), p.chunks, q.sm_count, &index, &splits);
-  p.chunks_per_split = (p.chunks + splits - 1) / splits;
-  switch (index) {
-    case 0: return int(LaunchTiles<16>(q, a, p, 0, splits));
-    case 1: return int(LaunchTiles<32>(q, a, p, 1, splits));
-    case 2: return int(LaunchTiles<64>(q, a, p, 2, splits));
-    case 3: return int(LaunchTiles<128>(q, a, p, 3, splits));
-    default: return int(LaunchWide(q, a, p));
+  const LinearTiling c = experts ? ChooseExpertLinear(a.slots.slots, a.slots.experts, a.slots.tile_rows, a.n, p.chunks, q.sm_count)
+                                 : ChooseLinear(a.t, a.n, a.heads, p.chunks, q.sm_count);
+  p.chunks_per_split = (p.chunks + c.splits - 1) / c.splits;
+  switch (c.index) {
+    case 0: return int(LaunchTiles<16>(q, a, p, 0, c.splits));
+    case 1: return int(LaunchTiles<32>(q, a, p, 1, c.splits));
+    case 2: return int(LaunchTiles<64>(q, a, p, 2, c.splits));
+    case 3: return int(LaunchTiles<128>(q, a, p, 3, c.splits));
+    default: return int(c.pair ? LaunchWide<true>(q, a, p) : LaunchWide<false>(q, a, p));
   }
 }
 
