@@ -81,3 +81,18 @@ def test_experts_of_many_rows(module, experts, top, plan_dir):
     else:
         config = module.model(264, 131, [module.latent(4, 32, 16, 32, 64, 48, mlp)], groups=2)
     check(module, config, module.weights_for(config, "bf16"), plan_dir, ([530], [300, 230]))
+
+
+# (experts, top, their gate and up rows together, or the up rows) whose products take tiles of 256 rows for 530 tokens of width 2056, as
+# test_linear_rules.py checks: less than a tile an expert, and just over one
+WIDE_EXPERTS = [(8, 2, 1800), (4, 2, 3000)]
+
+
+@pytest.mark.parametrize("module", [nadilorn_case, benarax_case], ids=["input weighted", "output weighted"])
+@pytest.mark.parametrize("experts,top,rows", WIDE_EXPERTS)
+def test_experts_on_wide_tiles(module, experts, top, rows, plan_dir):
+    if module is nadilorn_case:
+        config = module.model(2056, 131, [module.layer(4, 2, 32, 32, 16, 90, module.moe(experts, top, rows))])
+    else:
+        config = module.model(2056, 131, [module.latent(4, 32, 16, 32, 64, 48, module.moe(experts, top, rows // 2))], groups=2)
+    check(module, config, module.weights_for(config, "bf16"), plan_dir, ([530],))

@@ -21,7 +21,6 @@
 namespace tmb {
 namespace {
 
-constexpr int kStepK = 64;                  // 16-bit elements per 128-byte swizzle row
 constexpr int kWeightBytes = kRowsM * kStepK * 2;
 constexpr int kLinearThreads = 320;         // producer warp, issuing warp, eight epilogue warps
 
@@ -788,7 +787,9 @@ cudaError_t LaunchTiles(const Queue& q, const LinearArgs& a, const LinearParams&
 
 }  // namespace
 
-int ExpertTileRows(const Queue& q, int slots, int experts) { return q.f32 ? kTile32 : ExpertRows(slots, experts); }
+int ExpertTileRows(const Queue& q, int slots, int experts, int up, int width, int ff) {
+  return q.f32 ? kTile32 : ExpertRows(slots, experts, up, width, ff, q.sm_count);
+}
 
 int PrepareLinear() {
   cudaError_t err = RaiseLimit<16>();

@@ -5,6 +5,7 @@
 namespace tmb {
 
 constexpr int kRowsM = 128;                 // weight rows per tile
+constexpr int kStepK = 64;                  // 16-bit elements per 128-byte swizzle row
 constexpr int kWide = 256;                  // tokens of the widest tiles
 constexpr int kMaxCluster = 8;
 
@@ -42,12 +43,27 @@ inline LinearTiling ChooseLinear(int t, int n, int heads, int chunks, int sms) {
 // Most tiles of `tile_rows` that a step's slots can fall into: full ones, and one more for every expert in use.
 inline int MostExpertTiles(int slots, int experts, int tile_rows) { return slots / tile_rows + std::min(experts, slots); }
 
-// Slots per tile: an expert's on average; most experts have no more than 4/3 of it.
-inline int ExpertRows(int slots, int experts) {
+// Roughly what a product of n rows an expert over `chunks` of K takes in tiles of `rows` slots: rounds of tiles, a CTA an SM or two that share
+// one, by the rows a tile copies. (An expert's slots end where they end: half a tile more than they fill, but no less than one.)
+inline double ExpertCost(int slots, int experts, int rows, int n, int chunks, int sms) {
+  const double share = double(slots) / experts, each = std::max(1.0, share / rows + 0.5);
+  const double tiles = experts * each * ((n + kRowsM - 1) / kRowsM);
+  return Rounds((long long)(tiles), sms) * (kRowsM + share / each) * chunks * (rows == kWide ? 1.0 : 0.9);
+}
+
+// Slots per tile: an expert's on average; most experts have no more than 4/3 of it. 256 (linear_wide) where its rounds end before those of 128
+// (linear_tiles, two CTAs an SM, K split over the SMs that few tiles leave idle) for both products of an expert together: `up` rows over
+// `width` columns, `width` rows over `ff`. Both by 256 and by 128, us, width 2048: 128 experts of 1152, 128 slots each 311 / 359; 32 of 768, 250 slots
+// 114 / 140; 16 of 2048, 125 slots 92 / 110; but 8 of 512, 125 slots 49 / 38, 8 of 1024, 500 slots 95 / 76, 32 of 768, 125 slots 95 / 89.
+inline int ExpertRows(int slots, int experts, int up, int width, int ff, int sms) {
   const int share = (slots + experts - 1) / experts;
   int rows = 16;
   while (rows < kWide && rows * 3 < share * 4) rows *= 2;
-  return rows;
+  if (rows < kWide) return rows;
+  auto cost = [&](int of) {
+    return ExpertCost(slots, experts, of, up, (width + kStepK - 1) / kStepK, sms) + ExpertCost(slots, experts, of, width, (ff + kStepK - 1) / kStepK, sms);
+  };
+  return cost(kWide) <= cost(kWide / 2) ? kWide : kWide / 2;
 }
 
 // Per expert: the tile width is that of the slot table; K splits until the tiles to be expected cover the SMs.

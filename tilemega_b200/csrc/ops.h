@@ -199,7 +199,8 @@ struct LinearArgs {
   Glu glu;
   ExpertSlots slots;         // expert epilogues
 };
-int ExpertTileRows(const Queue& q, int slots, int experts);   // slots per tile that suits this many
+// Slots per tile that suits this many, of experts with `up` rows over `width` columns and `width` rows over `ff`.
+int ExpertTileRows(const Queue& q, int slots, int experts, int up, int width, int ff);
 int PrepareLinear();         // raises the kernels' shared-memory limits (once per device)
 bool EncodeLinear(LinearMaps* maps, const void* weight, uint64_t n, const void* activations, uint64_t rows, uint64_t k_stride);
 bool EncodeHeads(LinearMaps* maps, const void* weight, uint64_t n, uint64_t k_stride, const void* activations, uint64_t rows, uint64_t in_stride);

@@ -510,7 +510,7 @@ int Enqueue(RaggedPlan* plan, uint32_t entries, uint32_t rows, uint32_t longest,
       slots.experts = mlp.experts;
       slots.top = mlp.top;
       slots.slots = r.rows * mlp.top;
-      slots.tile_rows = ExpertTileRows(q, slots.slots, slots.experts);
+      slots.tile_rows = ExpertTileRows(q, slots.slots, slots.experts, mlp.output_weighted ? mlp.packed_rows() : mlp.ff, W, mlp.ff);
       RouteArgs a{};
       a.h = plan->normed;
       a.router = buffer(layer.router);
