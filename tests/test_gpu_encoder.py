@@ -93,10 +93,11 @@ def test_padded_sequences_match_the_oracle_and_the_module_fixture(plan_dir):
     assert (hidden - truth).abs().max().item() <= NOISE_FACTOR * (yard.float() - truth).abs().max().item() + 1e-3
 
 
-@pytest.mark.parametrize("batch,dtype_name", [(1, "f16"), (8, "f16"), (8, "bf16")])
+@pytest.mark.parametrize("batch,dtype_name", [(1, "f16"), (8, "f16"), (8, "bf16"), (28, "bf16"), (32, "f16")])
 def test_bert_base_shape_matches_the_oracle(batch, dtype_name, plan_dir):
     """The benchmark's shapes: 12 layers, hidden 768, 12 heads, FFN 3072, vocabulary 30522, batch x 128 tokens
-    (batch 1: 32-row weight tiles and K split in 4; batch 8: 128-row tiles, K split in 2)."""
+    (batch 1: 32-row weight tiles and K split in 4; batch 8: 128-row tiles, K split in 2, persistent tiles for FFN up, one a CTA; batches
+    28 and 32: persistent tiles 128, 192 and 256 wide, up to five a CTA, for every projection)."""
     run_case(synthetic.BERT_BASE, batch, dtype_name, plan_dir, seed=20)
 
 

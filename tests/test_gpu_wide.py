@@ -71,6 +71,14 @@ def test_pairs_that_would_take_a_round_more(plan_dir):
     check(case, config, case.weights_for(config, "bf16"), plan_dir, ([530],))
 
 
+@pytest.mark.parametrize("side", [5100, 6272])
+def test_side_inputs(side, plan_dir):
+    """Parts of the second embedding so wide that their gate runs on wide tiles, by pairs of CTAs and by single ones."""
+    case = benarax_case
+    config = case.model(96, 131, [case.latent(4, 32, 16, 32, 64, 48)], groups=2, side=side)
+    check(case, config, case.weights_for(config, "bf16"), plan_dir, ([530],))
+
+
 @pytest.mark.parametrize("module", [nadilorn_case, benarax_case], ids=["input weighted", "output weighted"])
 @pytest.mark.parametrize("experts,top", [(3, 2), (5, 1), (2, 2), (7, 3)])
 def test_experts_of_many_rows(module, experts, top, plan_dir):
