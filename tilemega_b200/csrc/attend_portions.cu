@@ -22,8 +22,7 @@ constexpr unsigned kWaitLoader = 0xA7700001u, kWaitMma = 0xA7700002u, kWaitSoftm
 template <int KC, int VC, int TILES> struct PortionShape {
   static constexpr int kThreads = 32 * 4 * (TILES + 1);
   static constexpr int kKeyStages = 2, kValueStages = KC > 2 && TILES > 1 ? 2 : 4;   // (values by half blocks)
-  static constexpr int kUsed = (TILES * KC + kKeyStages * KC) * kChunk + kValueStages * VC * kHalfChunk + 1024;
-  static constexpr int kSmem = kUsed > 120 * 1024 ? kUsed : 120 * 1024;      // (one CTA an SM: tensor memory is for one)
+  static constexpr int kSmem = (TILES * KC + kKeyStages * KC) * kChunk + kValueStages * VC * kHalfChunk + 1024;   // (registers allow one CTA an SM in any form)
   static constexpr int kColumns = TILES == 2 ? 512 : 256;
   static constexpr int kSums = 128 * TILES;                                  // first column of the weighted sums
 };
@@ -91,12 +90,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 // enter the second product from there, head and remainder one after the other: about 16 bits of every weight. What a row's
 // weights are relative to follows its maximum only in steps of 2^8, so that its sums are seldom scaled.
 //
-// Bound by the tensor pipe: an instruction of 128 x 128 x 16 leaves every 80 to 95 cycles (64 at peak, where no other product or
-// softmax is under way), and the remainders' products are half as much again as scores and sums need. 2048 tokens, 32 heads of
-// 128 over 8 key heads: 75 us where attend_tiles takes 337; 2048 tokens behind 4096, 32 heads of 192 and 128: 290 us for 1770
-// (300 GFLOP executed; two rounds of CTAs, 13 % of it the second one's end). What that took: keys by TMA instead of 16-byte copies of
-// three warps (11000 cycles a block went into issuing those, 98 and 518 us), a warp that stays together around the issuing lane
-// (90 and 340 us without), values by half blocks where shared memory holds just one, output rows written by eight lanes each.
+// Bound by the tensor pipe and the softmax between its two products: the pipe is active half of the time behind 4096 positions, 30 % at 2048
+// rows from the start, where a CTA's start and end weigh more; a third of the products are the remainders'. 2048 tokens, 32 heads of
+// 128 over 8 key heads: 75 us where attend_tiles takes 337; 2048 tokens behind 4096, 32 heads of 192 and 128: 290 us for 1770 (300 GFLOP executed;
+// two rounds of CTAs). What that took: keys by TMA instead of 16-byte copies of three warps (98 and 518 us with those), a warp that stays together
+// around the issuing lane (90 and 340 without), values by half blocks where shared memory holds just one, output rows written by eight lanes each.
 template <int KC, int VC, int TILES>
 __global__ void __launch_bounds__(PortionShape<KC, VC, TILES>::kThreads, 1) attend_portions(StepRows r, AttendParams p, const __grid_constant__ CUtensorMap k_map,
                                                                                            const __grid_constant__ CUtensorMap v_map, unsigned* status, bool vector_rows) {
@@ -459,8 +457,9 @@ int LaunchPortions(const Queue& q, const StepRows& r, const AttendParams& p, con
 
 template <int KC, int VC> int PortionsWith(const Queue& q, const StepRows& r, const AttendParams& p, const CUtensorMap& k_map, const CUtensorMap& v_map) {
   const int per_tile = 128 / p.sub_heads, tiles = (r.longest + per_tile - 1) / per_tile;
-  // Two tiles a CTA share its keys and overlap one's softmax with the other's products: a pair takes about 1.6 times as long
-  // as a tile alone. One tile each where that ends sooner all the same, for want of CTAs.
+  // Two tiles a CTA share its keys and overlap one's softmax with the other's products. Where both ways are one round of CTAs, two take
+  // 1.1 to 1.2 times as long as one (8B shape, 431 rows 33 us for 30, behind 2000 67 for 59; 16 heads of 192, 1000 rows 68 for 58): one tile
+  // each. At half the rounds 0.6 to 0.9 times (2048 rows 75 for 125, 1000 rows 43 for 53; 32 heads of 192, 700 rows 42 for 47): two.
   const int units = p.kv_heads * p.subs * std::max(1, r.entries - r.singles);
   auto rounds = [&](int count) { return (count + q.sm_count - 1) / q.sm_count; };
   if (16 * rounds((tiles + 1) / 2 * units) <= 10 * rounds(tiles * units)) return LaunchPortions<KC, VC, 2>(q, r, p, k_map, v_map, tiles);

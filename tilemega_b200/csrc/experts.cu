@@ -1,5 +1,8 @@
-// Routing of a ragged step's rows to experts: router logits, the best experts of every row, and the assignments sorted
-// by expert into the tiles the per-expert products run on. One kernel: its last CTA to finish sorts.
+// Routing of a ragged step's rows to experts: router logits, the best experts of every row, and the assignments in order of
+// expert, cut into the tiles the per-expert products run on. Up to 64 rows one kernel does all of it and its last CTA sorts; for more rows
+// the logits are there already, and where the products read rows put in order (bf16, tiles of more than kGatherRows) assignments take
+// their place among their expert's as they are chosen: the last CTA only lays the experts out, and scatter_rows fills the table of
+// slots as it copies the rows. Otherwise the last CTA sorts there too.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -280,7 +283,7 @@ __device__ __forceinline__ bool arrives_last(unsigned* counter, unsigned of, uns
 
 // FUSED: blockIdx = (eight experts, eight rows); a warp runs its expert's router row over the rows, the last CTA of the
 // rows chooses, a warp a row, and the last of all sorts. Otherwise the logits are there, a warp chooses for one row, and
-// the last CTA sorts.
+// the last CTA sorts, or with ranks (RouteArgs::rank) only lays the experts out.
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(FUSED ? 256 : 1024) route(RouteArgs a) {
   __shared__ int counts[kMaxExperts], first[kMaxExperts];

@@ -1,11 +1,12 @@
 // Matrix products of a ragged step: D[t][n] = sum_k activations[t][k] weight[n][k] for any t, n and k.
 //
-// bf16: weights fill the M side of a tcgen05 tile (128 weight rows), the step's tokens the N side (16 .. 256), so one
-// kernel serves a single decoded token (a weight stream: many small stages in flight, K split over the CTAs of a
-// cluster, whose partial tiles meet in distributed shared memory) and a prompt of thousands (128 x 256 tiles). Both
-// operands arrive by TMA in 128-byte-swizzled stages; weight tiles of the first stages are requested before the
-// dependency wait. A thread of the epilogue owns one weight row (output feature), so a warp's stores are runs of 32
-// consecutive features of one token. fp32: a tiled kernel of plain fused multiply-adds.
+// bf16: weights fill the M side of a tcgen05 tile (128 weight rows, 256 over a pair of CTAs), the step's tokens the N side. linear_tiles,
+// 16 .. 128 tokens, serves a single decoded token (a weight stream: many small stages in flight, K split over the CTAs of a
+// cluster, whose partial tiles meet in distributed shared memory) up to small batches; linear_wide, 256 tokens and a CTA or a pair
+// that takes tile after tile, prompts of thousands and experts of many rows. Both operands arrive by TMA in 128-byte-swizzled
+// stages; weight tiles of the first stages are requested before the dependency wait. A thread of the epilogue owns one weight row
+// (output feature), so a warp's stores are runs of 32 consecutive features of one token. fp32: a tiled kernel of plain fused
+// multiply-adds. Which of them a product takes is in linear_rules.h.
 #include <cuda_bf16.h>
 
 #include <algorithm>
