@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(PortionShape<KC, VC, TILES>::kThreads, 1) atte
       __syncwarp();
       // (also behind a wait that gave up: tensor memory is freed once no product runs)
       for (int t = 0; t < TILES; ++t) drained(&o_full[t], 0);
+      __syncwarp();
     }
   } else {
     if constexpr (TILES == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
@@ -442,7 +443,10 @@ __global__ void __launch_bounds__(PortionShape<KC, VC, TILES>::kThreads, 1) atte
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 4 * TILES) tmem_dealloc(tmem, Shape::kColumns);
+  if (warp == 4 * TILES) {
+    __syncwarp();
+    tmem_dealloc(tmem, Shape::kColumns);
+  }
 }
 
 template <int KC, int VC, int TILES>

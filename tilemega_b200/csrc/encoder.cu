@@ -345,7 +345,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) encoder_wide(const __grid_con
           if (elect_one()) umma_commit(&sum_full[b]);
           __syncwarp();
         },
-        [&](int b, uint32_t parity) { drained(&sum_full[b], parity); });
+        [&](int b, uint32_t parity) {
+          drained(&sum_full[b], parity);
+          __syncwarp();
+        });
   } else {
     const int quarter = warp & 3, column_half = (warp - 2) >> 2;
     write_tiles(
@@ -382,6 +385,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) encoder_wide(const __grid_con
   __syncthreads();
   if (warp == 1) {
     tcgen05_fence_after();
+    __syncwarp();
     tmem_dealloc(tmem, 2 * A);
   }
 }

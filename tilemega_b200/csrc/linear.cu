@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(kLinearThreads) linear_tiles(const __grid_cons
   __syncthreads();
   if (warp == 1) {
     tcgen05_fence_after();
+    __syncwarp();
     tmem_dealloc(tmem, Shape::kTmemCols);
   }
 }
@@ -521,7 +522,10 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
           }
           __syncwarp();
         },
-        [&](int b, uint32_t parity) { drained(&sum_full[b], parity); });
+        [&](int b, uint32_t parity) {
+          drained(&sum_full[b], parity);
+          __syncwarp();
+        });
   } else {
     const int quarter = warp & 3, column_half = (warp - 2) >> 2;
     write_tiles(
@@ -618,9 +622,11 @@ __global__ void __launch_bounds__(kLinearThreads, 1) linear_wide(const __grid_co
   }
   if (warp == 1) {
     tcgen05_fence_after();
+    __syncwarp();
     if constexpr (PAIR) tmem_dealloc_pair(tmem, 512);
     else tmem_dealloc(tmem, 512);
   }
+  if constexpr (PAIR) cluster_sync();                    // (both free it together: neither is gone before the other has)
 }
 
 // ---- fp32 --------------------------------------------------------------------------------------------------------
